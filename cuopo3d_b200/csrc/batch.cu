@@ -20,41 +20,12 @@
 #include <type_traits>
 #include <vector>
 
+#include "batch_device.cuh"
 #include "pass_body.cuh"
 #include "tpass_line.cuh"
 #include "solver_internal.h"
 
 namespace opo {
-
-// One launch's share of a descriptor array: instances [first, first + ninst) with their
-// tile prefix at prefix[pfirst ...] (starting at 0), total_tiles tiles.
-struct BatchHeader {
-    unsigned ninst;
-    unsigned total_tiles;
-    unsigned first;
-    unsigned pfirst;
-};
-
-template <typename Args> __host__ __device__ constexpr unsigned desc_bytes() { return (unsigned)((sizeof(Args) + 127) / 128 * 128); }
-
-template <typename Args> __device__ __forceinline__ void stage_desc(const Args *src, Args *dst)
-{
-    const unsigned *s = reinterpret_cast<const unsigned *>(src);
-    unsigned *d = reinterpret_cast<unsigned *>(dst);
-    for (unsigned k = threadIdx.x; k < sizeof(Args) / 4; k += blockDim.x) d[k] = s[k];
-}
-
-// Largest i < ninst with prefix[i] <= gt.
-__device__ __forceinline__ int find_inst(const unsigned *prefix, unsigned ninst, unsigned gt)
-{
-    int lo = 0, hi = (int)ninst - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(prefix + mid) <= gt) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
 
 template <typename C, int R1, int THREADS, int RMAX>
 __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 4 : 1)
@@ -208,7 +179,10 @@ inline int t_group(PassVariant v, int line_nt)
     if (!is_line(v)) return 3;
     return line_nt == 256 ? 0 : line_nt == 128 ? 1 : line_nt == 64 ? 2 : 3;
 }
-constexpr int kLineGroupNT[3] = {256, 128, 64};
+
+// x and y groups: the instances whose axis length has a compiled body (axis_line.cuh; one
+// kernel holds every body) and the rest.
+constexpr int kAxGroups = 2;
 
 template <typename C> bool batch_t_generic_func(PassVariant v, const void **fn);
 
@@ -292,18 +266,22 @@ struct OpoBatch {
     // device state
     void *d_t[3] = {};       // t descriptors: first, middle, final
     void *d_ax[2][2] = {};   // [x, y][crystal, free]
-    unsigned *d_prefix[3] = {};  // t: one prefix per t-pass group, back to back
-    opo::BatchHeader *d_hdr = nullptr;  // [t-pass groups..., x, y]
+    unsigned *d_prefix[3] = {};  // one prefix per group of the pass, back to back
+    opo::BatchHeader *d_hdr = nullptr;  // [t-pass groups..., x groups, y groups]
     opo::SlotFields *d_slotf = nullptr;
     double *d_partials = nullptr, *d_sums = nullptr;
     std::vector<unsigned char> h_desc;  // host staging
     bool dirty = true;
     std::vector<char> last_flag;  // per order position: on its last round trip when uploaded
     cudaGraphExec_t graph = nullptr;
-    size_t graph_smem[3] = {0, 0, 0};  // t: the generic group's
-    int grid[3] = {0, 0, 0};
-    int t_grid[opo::kTGroups] = {};
-    size_t t_smem[opo::kTGroups] = {};
+    // launch configuration of every group in the graph (groups without instances when the
+    // graph was built are not in it: their first instance rebuilds it)
+    struct Group {
+        bool on = false;
+        int grid = 0;
+        size_t smem = 0;  // the largest tile of the group's instances
+    };
+    Group t_group[opo::kTGroups], ax_group[2][opo::kAxGroups];
     long long launches = 0;
     int launches_rt = 0;
     std::string err;
@@ -330,6 +308,8 @@ int bfail(OpoBatch *b, int code, const std::string &msg)
 
 bool slot_ok(const OpoBatch *b, int slot) { return b && slot >= 0 && slot < b->capacity && b->slots[slot].used; }
 
+int ax_group_of(const OpoSolver *s, int kind) { return opo::solver_line_n(s, kind) ? 0 : 1; }
+
 template <typename C> int upload_descriptors(OpoBatch *b)
 {
     using TA = opo::TPassArgs<C>;
@@ -340,7 +320,6 @@ template <typename C> int upload_descriptors(OpoBatch *b)
     std::vector<unsigned> prefix[3];
     std::vector<opo::SlotFields> sf;
     std::vector<int> tgroup;
-    for (int k = 1; k < 3; k++) prefix[k].push_back(0);
     b->last_flag.assign(n, 0);
     for (int pos = 0; pos < n; pos++) {
         Slot &sl = b->slots[b->order[pos]];
@@ -363,19 +342,13 @@ template <typename C> int upload_descriptors(OpoBatch *b)
             ax[a][1].push_back(opo::make_axis_args<C>(s, 1 + a, 1, (diff && !last) ? 6u : 0u));
         }
         tgroup.push_back(opo::t_group(b->v[0], opo::solver_line_nt(s)));
-        for (int k = 1; k < 3; k++) {
-            int nt;
-            size_t sm;
-            opo::solver_pass_info(s, k, &nt, &sm);
-            prefix[k].push_back(prefix[k].back() + (unsigned)nt);
-        }
         opo::SlotFields f;
         for (int k = 0; k < 3; k++) f.f[k] = opo::solver_field(s, k + 1);
         f.n = (unsigned long long)sl.voxels;
         sf.push_back(f);
     }
     // t descriptors group-major, each group with its own tile prefix (from 0)
-    opo::BatchHeader hdr[opo::kTGroups + 2];
+    opo::BatchHeader hdr[opo::kTGroups + 2 * opo::kAxGroups];
     {
         std::vector<TA> ts[3];
         for (int g = 0; g < opo::kTGroups; g++) {
@@ -395,6 +368,29 @@ template <typename C> int upload_descriptors(OpoBatch *b)
         }
         for (int k = 0; k < 3; k++) t[k].swap(ts[k]);
     }
+    // x and y descriptors likewise
+    for (int a = 0; a < 2; a++) {
+        std::vector<AA> as[2];
+        std::vector<unsigned> &pre = prefix[1 + a];
+        for (int g = 0; g < opo::kAxGroups; g++) {
+            opo::BatchHeader &h = hdr[opo::kTGroups + a * opo::kAxGroups + g];
+            h.first = (unsigned)as[0].size();
+            h.pfirst = (unsigned)pre.size();
+            pre.push_back(0);
+            for (int pos = 0; pos < n; pos++) {
+                const OpoSolver *s = b->slots[b->order[pos]].s;
+                if (ax_group_of(s, 1 + a) != g) continue;
+                for (int w = 0; w < 2; w++) as[w].push_back(ax[a][w][pos]);
+                int nt;
+                size_t sm;
+                opo::solver_pass_info(s, 1 + a, &nt, &sm);
+                pre.push_back(pre.back() + (unsigned)nt);
+            }
+            h.ninst = (unsigned)as[0].size() - h.first;
+            h.total_tiles = pre.back();
+        }
+        for (int w = 0; w < 2; w++) ax[a][w].swap(as[w]);
+    }
     const size_t cap = (size_t)b->capacity;
     for (int k = 0; k < 3; k++)
         if (n) OPO_BCU(b, cudaMemcpyAsync(b->d_t[k], t[k].data(), sizeof(TA) * n, cudaMemcpyHostToDevice, b->stream), "descriptors");
@@ -404,7 +400,6 @@ template <typename C> int upload_descriptors(OpoBatch *b)
     for (int k = 0; k < 3; k++)
         OPO_BCU(b, cudaMemcpyAsync(b->d_prefix[k], prefix[k].data(), sizeof(unsigned) * prefix[k].size(),
                                    cudaMemcpyHostToDevice, b->stream), "prefix");
-    for (int a = 0; a < 2; a++) hdr[opo::kTGroups + a] = opo::BatchHeader{(unsigned)n, prefix[1 + a].back(), 0, 0};
     OPO_BCU(b, cudaMemcpyAsync(b->d_hdr, hdr, sizeof(hdr), cudaMemcpyHostToDevice, b->stream), "header");
     if (n) OPO_BCU(b, cudaMemcpyAsync(b->d_slotf, sf.data(), sizeof(opo::SlotFields) * n, cudaMemcpyHostToDevice, b->stream), "slot fields");
     // pageable sources: make the copies complete before the host vectors go away
@@ -422,29 +417,43 @@ int persistent_grid(OpoBatch *b, const void *fn, int threads, size_t smem)
     return b->sms * per;
 }
 
+// Kernels of every group: t-pass groups, and per axis the line bodies and the generic body.
+template <typename C> struct BatchFuncs {
+    const void *t[opo::kTGroups];
+    const void *ax[2][opo::kAxGroups];
+    int ax_threads[2][opo::kAxGroups];
+};
+
+template <typename C> bool batch_funcs(const OpoBatch *b, BatchFuncs<C> &f)
+{
+    if (!opo::batch_t_funcs<C>(b->v[0], f.t) || !opo::batch_a_func<C>(b->v[1], true, &f.ax[0][1]) ||
+        !opo::batch_a_func<C>(b->v[2], false, &f.ax[1][1]))
+        return false;
+    f.ax[0][0] = opo::axis_line_batch_func<C, true>(&f.ax_threads[0][0]);
+    f.ax[1][0] = opo::axis_line_batch_func<C, false>(&f.ax_threads[1][0]);
+    for (int a = 0; a < 2; a++) f.ax_threads[a][1] = b->v[1 + a].threads;
+    return true;
+}
+
 template <typename C> int enqueue_batch_round_trip(OpoBatch *b)
 {
     using TA = opo::TPassArgs<C>;
     using AA = opo::AxisArgs<C>;
-    const void *ft[opo::kTGroups], *fx = nullptr, *fy = nullptr;
-    if (!opo::batch_t_funcs<C>(b->v[0], ft) || !opo::batch_a_func<C>(b->v[1], true, &fx) ||
-        !opo::batch_a_func<C>(b->v[2], false, &fy))
-        return bfail(b, OPO_ERR_INVALID, "batch kernel variant not compiled");
-    const size_t sx = opo::desc_bytes<AA>() + b->graph_smem[1];
-    const size_t sy = opo::desc_bytes<AA>() + b->graph_smem[2];
+    BatchFuncs<C> f;
+    if (!batch_funcs<C>(b, f)) return bfail(b, OPO_ERR_INVALID, "batch kernel variant not compiled");
     const opo::BatchHeader *hdr = b->d_hdr;
-    // one launch per t-pass group the setting populates; a group without instances
-    // (its header counts none) returns at once
+    // one launch per group that has (or had, when the graph was built) instances; a group
+    // without any (its header counts none) returns at once
     auto launch_t = [&](int which, int tp) -> cudaError_t {
         const TA *descs = static_cast<const TA *>(b->d_t[which]);
         const unsigned *pre = b->d_prefix[0];
         for (int g = 0; g < opo::kTGroups; g++) {
-            if (!ft[g]) continue;
+            if (!b->t_group[g].on) continue;
             const opo::BatchHeader *h = hdr + g;
             void *args[] = {(void *)&descs, (void *)&pre, (void *)&h, (void *)&tp};
             b->launches++;
-            cudaError_t e = cudaLaunchKernel(ft[g], dim3(b->t_grid[g]), dim3(b->v[0].threads), args, b->t_smem[g],
-                                             b->stream);
+            cudaError_t e = cudaLaunchKernel(f.t[g], dim3(b->t_group[g].grid), dim3(b->v[0].threads), args,
+                                             b->t_group[g].smem, b->stream);
             if (e != cudaSuccess) return e;
         }
         return cudaSuccess;
@@ -452,11 +461,17 @@ template <typename C> int enqueue_batch_round_trip(OpoBatch *b)
     auto launch_a = [&](int axis, int which) -> cudaError_t {
         const AA *descs = static_cast<const AA *>(b->d_ax[axis][which]);
         const unsigned *pre = b->d_prefix[1 + axis];
-        const opo::BatchHeader *h = hdr + opo::kTGroups + axis;
-        void *args[] = {(void *)&descs, (void *)&pre, (void *)&h};
-        b->launches++;
-        return cudaLaunchKernel(axis == 0 ? fx : fy, dim3(b->grid[1 + axis]), dim3(b->v[1 + axis].threads), args,
-                                axis == 0 ? sx : sy, b->stream);
+        for (int g = 0; g < opo::kAxGroups; g++) {
+            const OpoBatch::Group &gr = b->ax_group[axis][g];
+            if (!gr.on) continue;
+            const opo::BatchHeader *h = hdr + opo::kTGroups + axis * opo::kAxGroups + g;
+            void *args[] = {(void *)&descs, (void *)&pre, (void *)&h};
+            b->launches++;
+            cudaError_t e = cudaLaunchKernel(f.ax[axis][g], dim3(gr.grid), dim3(f.ax_threads[axis][g]), args, gr.smem,
+                                             b->stream);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
     };
     for (int k = 0; k < b->n_steps; k++) {
         OPO_BCU(b, launch_t(k == 0 ? 0 : 1, k), "batch t-pass");
@@ -469,47 +484,57 @@ template <typename C> int enqueue_batch_round_trip(OpoBatch *b)
     return OPO_OK;
 }
 
+// Whether the graph covers the resident instances: their groups, and their tiles' shared
+// memory.  With grow, the group configuration is extended to what they need.
+bool graph_covers(OpoBatch *b, bool grow)
+{
+    bool ok = true;
+    auto need = [&](OpoBatch::Group &g, size_t smem) {
+        if (g.on && smem <= g.smem) return;
+        ok = false;
+        if (!grow) return;
+        g.on = true;
+        g.smem = std::max(g.smem, smem);
+    };
+    for (int sidx : b->order) {
+        const OpoSolver *s = b->slots[sidx].s;
+        int nt;
+        size_t sm;
+        opo::solver_pass_info(s, 0, &nt, &sm);
+        const size_t dt = b->precision == OPO_FP64 ? opo::desc_bytes<opo::TPassArgs<double2>>()
+                                                   : opo::desc_bytes<opo::TPassArgs<float2>>();
+        const size_t da = b->precision == OPO_FP64 ? opo::desc_bytes<opo::AxisArgs<double2>>()
+                                                   : opo::desc_bytes<opo::AxisArgs<float2>>();
+        need(b->t_group[opo::t_group(b->v[0], opo::solver_line_nt(s))], dt + sm);
+        for (int a = 0; a < 2; a++) {
+            opo::solver_pass_info(s, 1 + a, &nt, &sm);
+            need(b->ax_group[a][ax_group_of(s, 1 + a)], da + sm);
+        }
+    }
+    return ok;
+}
+
 template <typename C> int build_batch_graph(OpoBatch *b)
 {
-    using TA = opo::TPassArgs<C>;
-    using AA = opo::AxisArgs<C>;
     if (b->graph) {
         cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
     }
-    // shared memory: the largest tile of any slot, per pass kind (t: of the slots in the
-    // generic group; a line body's tile has a fixed size)
-    for (int k = 0; k < 3; k++) b->graph_smem[k] = 0;
-    for (int sidx : b->order) {
-        for (int k = 0; k < 3; k++) {
-            int nt;
-            size_t sm;
-            opo::solver_pass_info(b->slots[sidx].s, k, &nt, &sm);
-            if (k == 0 && opo::t_group(b->v[0], opo::solver_line_nt(b->slots[sidx].s)) != 3) continue;
-            b->graph_smem[k] = std::max(b->graph_smem[k], sm);
-        }
-    }
-    const void *ft[opo::kTGroups], *fx = nullptr, *fy = nullptr;
-    if (!opo::batch_t_funcs<C>(b->v[0], ft) || !opo::batch_a_func<C>(b->v[1], true, &fx) ||
-        !opo::batch_a_func<C>(b->v[2], false, &fy))
-        return bfail(b, OPO_ERR_INVALID, "batch kernel variant not compiled");
-    const bool fp64 = sizeof(C) == 16;
-    for (int g = 0; g < opo::kTGroups; g++) {
-        if (!ft[g]) continue;
-        b->t_smem[g] = opo::desc_bytes<TA>() +
-                       (g < 3 ? opo::tpass_line_smem(fp64, opo::kLineGroupNT[g], opo::line_radix(opo::kLineGroupNT[g]))
-                              : b->graph_smem[0]);
-        if (b->t_smem[g] > 227 * 1024) return bfail(b, OPO_ERR_INVALID, "batched tile does not fit in shared memory");
-        OPO_BCU(b, cudaFuncSetAttribute(ft[g], cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024), "attribute");
-        b->t_grid[g] = persistent_grid(b, ft[g], b->v[0].threads, b->t_smem[g]);
-    }
-    const size_t sm[3] = {0, opo::desc_bytes<AA>() + b->graph_smem[1], opo::desc_bytes<AA>() + b->graph_smem[2]};
-    const void *fns[3] = {nullptr, fx, fy};
-    for (int k = 1; k < 3; k++) {
-        if (sm[k] > 227 * 1024) return bfail(b, OPO_ERR_INVALID, "batched tile does not fit in shared memory");
-        OPO_BCU(b, cudaFuncSetAttribute(fns[k], cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024), "attribute");
-        b->grid[k] = persistent_grid(b, fns[k], b->v[k].threads, sm[k]);
-    }
+    graph_covers(b, true);
+    BatchFuncs<C> f;
+    if (!batch_funcs<C>(b, f)) return bfail(b, OPO_ERR_INVALID, "batch kernel variant not compiled");
+    auto configure = [&](OpoBatch::Group &g, const void *fn, int threads) -> int {
+        if (!g.on) return OPO_OK;
+        if (g.smem > 227 * 1024) return bfail(b, OPO_ERR_INVALID, "batched tile does not fit in shared memory");
+        OPO_BCU(b, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024), "attribute");
+        g.grid = persistent_grid(b, fn, threads, g.smem);
+        return OPO_OK;
+    };
+    for (int g = 0; g < opo::kTGroups; g++)
+        if (int rc = configure(b->t_group[g], f.t[g], b->v[0].threads)) return rc;
+    for (int a = 0; a < 2; a++)
+        for (int g = 0; g < opo::kAxGroups; g++)
+            if (int rc = configure(b->ax_group[a][g], f.ax[a][g], f.ax_threads[a][g])) return rc;
     cudaGraph_t g = nullptr;
     OPO_BCU(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
     const long long before = b->launches;
@@ -541,16 +566,7 @@ template <typename C> int batch_run(OpoBatch *b, int n)
             int rc = upload_descriptors<C>(b);
             if (rc) return rc;
         }
-        bool rebuild = !b->graph;
-        for (int sidx : b->order)
-            for (int k = 0; k < 3; k++) {
-                int nt;
-                size_t sm;
-                opo::solver_pass_info(b->slots[sidx].s, k, &nt, &sm);
-                if (k == 0 && opo::t_group(b->v[0], opo::solver_line_nt(b->slots[sidx].s)) != 3) continue;
-                if (sm > b->graph_smem[k]) rebuild = true;
-            }
-        if (rebuild) {
+        if (!b->graph || !graph_covers(b, false)) {
             int rc = build_batch_graph<C>(b);
             if (rc) return rc;
         }
@@ -631,10 +647,10 @@ int opo_batch_create(int precision, int capacity, size_t hbm_budget, const int t
             for (int w = 0; w < 2 && !rc; w++)
                 if (cudaMalloc(&b->d_ax[a][w], asz * capacity) != cudaSuccess) rc = OPO_ERR_NOMEM;
         for (int k = 0; k < 3 && !rc; k++)
-            if (cudaMalloc((void **)&b->d_prefix[k], sizeof(unsigned) * (capacity + opo::kTGroups)) != cudaSuccess)
+            if (cudaMalloc((void **)&b->d_prefix[k], sizeof(unsigned) * (capacity + opo::kTGroups + opo::kAxGroups)) != cudaSuccess)
                 rc = OPO_ERR_NOMEM;
         if (rc) break;
-        if (cudaMalloc((void **)&b->d_hdr, sizeof(opo::BatchHeader) * (opo::kTGroups + 2)) != cudaSuccess ||
+        if (cudaMalloc((void **)&b->d_hdr, sizeof(opo::BatchHeader) * (opo::kTGroups + 2 * opo::kAxGroups)) != cudaSuccess ||
             cudaMalloc((void **)&b->d_slotf, sizeof(opo::SlotFields) * capacity) != cudaSuccess ||
             cudaMalloc((void **)&b->d_partials, sizeof(double) * 3 * opo::kTallyBlocks * capacity) != cudaSuccess ||
             cudaMalloc((void **)&b->d_sums, sizeof(double) * 3 * capacity) != cudaSuccess) {

@@ -47,7 +47,10 @@ inline std::vector<double> fp32_pair_compensation(const AxisPlan &pl, const std:
     butterfly_sq<2>(b2[2]);
     butterfly_sq<3>(b2[3]);
     butterfly_sq<4>(b2[4]);
+    butterfly_sq<6>(b2[6]);
     butterfly_sq<8>(b2[8]);
+    butterfly_sq<9>(b2[9]);
+    butterfly_sq<12>(b2[12]);
     butterfly_sq<16>(b2[16]);
     auto w2 = [&](int s, int k, int j) {
         if (k == 0) return 1.0;

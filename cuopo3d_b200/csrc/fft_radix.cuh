@@ -91,12 +91,15 @@ template <int S, typename C, typename T> __host__ __device__ __forceinline__ C c
     return S > 0 ? C{a.x * c - a.y * s, a.x * s + a.y * c} : C{a.x * c + a.y * s, a.y * c - a.x * s};
 }
 
-// Root-of-unity constants (values of cos and sin at multiples of pi/8 and pi/3).
+// Root-of-unity constants (values of cos and sin at multiples of pi/8, pi/3 and 2 pi/9).
 template <typename T> struct Roots {
     static constexpr T r2 = T(0.70710678118654752440);  // cos(pi/4)
     static constexpr T c8 = T(0.92387953251128675613);  // cos(pi/8)
     static constexpr T s8 = T(0.38268343236508977173);  // sin(pi/8)
     static constexpr T s3 = T(0.86602540378443864676);  // sin(pi/3)
+    static constexpr T c9 = T(0.76604444311897803520), s9 = T(0.64278760968653932632);      // 2 pi / 9
+    static constexpr T c9_2 = T(0.17364817766693034885), s9_2 = T(0.98480775301220805937);  // 4 pi / 9
+    static constexpr T c9_4 = T(-0.93969262078590838405), s9_4 = T(0.34202014332566873304);  // 8 pi / 9
 };
 
 template <int S, typename C> __host__ __device__ __forceinline__ void dft2(C &a, C &b)
@@ -137,6 +140,62 @@ template <int S, typename C> struct Dft<3, S, C> {
 
 template <int S, typename C> struct Dft<4, S, C> {
     __host__ __device__ __forceinline__ static void run(C *x) { dft4<S>(x[0], x[1], x[2], x[3]); }
+};
+
+// 6 = 2 x 3 and 12 = 4 x 3 by the prime-factor map (Good 1958): with coprime factors
+// n = 3 n2 + M n1 (mod 3 M), k = k1 mod 3 = k2 mod M separates the transform with no twiddles.
+template <int M, int S, typename C> __host__ __device__ __forceinline__ void dft_3xm(C *x)
+{
+    constexpr int N = 3 * M, E = M == 4 ? 9 : 3;  // E: 1 mod M, 0 mod 3;  4: 1 mod 3, 0 mod M
+    C y[N];
+#pragma unroll
+    for (int n2 = 0; n2 < M; n2++) {
+        C t[3] = {x[3 * n2 % N], x[(M + 3 * n2) % N], x[(2 * M + 3 * n2) % N]};
+        Dft<3, S, C>::run(t);
+        y[n2] = t[0];
+        y[M + n2] = t[1];
+        y[2 * M + n2] = t[2];
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < 3; k1++) {
+        Dft<M, S, C>::run(y + M * k1);
+#pragma unroll
+        for (int k2 = 0; k2 < M; k2++) x[(4 * k1 + E * k2) % N] = y[M * k1 + k2];
+    }
+}
+template <int S, typename C> struct Dft<6, S, C> {
+    __host__ __device__ __forceinline__ static void run(C *x) { dft_3xm<2, S>(x); }
+};
+template <int S, typename C> struct Dft<12, S, C> {
+    __host__ __device__ __forceinline__ static void run(C *x) { dft_3xm<4, S>(x); }
+};
+
+// 9 = 3 x 3: u_{m,r} = DFT3_j(x_{m+3j})_r, u_{m,r} *= W9^{m r}, y_{3k+r} = DFT3_m(u_{m,r})_k
+template <int S, typename C> struct Dft<9, S, C> {
+    __host__ __device__ __forceinline__ static void run(C *x)
+    {
+        using T = decltype(x[0].x);
+        using K = Roots<T>;
+        C u[3][3];  // [r][m]
+#pragma unroll
+        for (int m = 0; m < 3; m++) {
+            C t[3] = {x[m], x[m + 3], x[m + 6]};
+            Dft<3, S, C>::run(t);
+            u[0][m] = t[0];
+            u[1][m] = t[1];
+            u[2][m] = t[2];
+        }
+        u[1][1] = cmul_cs<S>(u[1][1], K::c9, K::s9);      // W^1
+        u[1][2] = cmul_cs<S>(u[1][2], K::c9_2, K::s9_2);  // W^2
+        u[2][1] = cmul_cs<S>(u[2][1], K::c9_2, K::s9_2);  // W^2
+        u[2][2] = cmul_cs<S>(u[2][2], K::c9_4, K::s9_4);  // W^4
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            Dft<3, S, C>::run(u[r]);
+#pragma unroll
+            for (int k = 0; k < 3; k++) x[3 * k + r] = u[r][k];
+        }
+    }
 };
 
 // 8 = 2 x 4: a_m = x_m + x_{m+4}, b_m = (x_m - x_{m+4}) W8^m, y_{2k} = DFT4(a), y_{2k+1} = DFT4(b)

@@ -3,6 +3,7 @@
 // cavity round trip (captured as CUDA graphs), and the C-ABI of include/cuopo3d.h.
 
 #include "../../include/cuopo3d.h"
+#include "axis_line.cuh"
 #include "fft_gain.h"
 #include "opo_internal.h"
 #include "solver_internal.h"
@@ -219,19 +220,9 @@ bool split_pow2(int e, int rmax, std::vector<int> &out)
     return true;
 }
 
-// Plan for n = 2^a 3^b with first-stage radix r1 (a power of two >= 4 dividing n, with
-// at least one more stage after it) and every other radix <= rmax.
-bool build_plan(int n, int r1, int rmax, opo::AxisPlan &p, std::vector<cd> &tw)
+// Plan of n points with the given stage radices (first stage first), and its twiddles.
+bool plan_of_radices(int n, const std::vector<int> &rad, opo::AxisPlan &p, std::vector<cd> &tw)
 {
-    if (n < 8 || r1 < 4 || (r1 & (r1 - 1)) || n % r1 || n / r1 < 2) return false;
-    int a = 0, b = 0, m = n / r1;
-    while (m % 2 == 0) { m /= 2; a++; }
-    while (m % 3 == 0) { m /= 3; b++; }
-    if (m != 1) return false;
-    std::vector<int> rad;
-    rad.push_back(r1);
-    for (int k = 0; k < b; k++) rad.push_back(3);
-    if (!split_pow2(a, rmax, rad)) return false;
     if (rad.size() < 2 || (int)rad.size() > opo::kMaxStages) return false;
     p = opo::AxisPlan{};
     p.n = n;
@@ -249,6 +240,22 @@ bool build_plan(int n, int r1, int rmax, opo::AxisPlan &p, std::vector<cd> &tw)
         L = q;
     }
     return L == 1;
+}
+
+// Plan for n = 2^a 3^b with first-stage radix r1 (a power of two >= 4 dividing n, with
+// at least one more stage after it) and every other radix <= rmax.
+bool build_plan(int n, int r1, int rmax, opo::AxisPlan &p, std::vector<cd> &tw)
+{
+    if (n < 8 || r1 < 4 || (r1 & (r1 - 1)) || n % r1 || n / r1 < 2) return false;
+    int a = 0, b = 0, m = n / r1;
+    while (m % 2 == 0) { m /= 2; a++; }
+    while (m % 3 == 0) { m /= 3; b++; }
+    if (m != 1) return false;
+    std::vector<int> rad;
+    rad.push_back(r1);
+    for (int k = 0; k < b; k++) rad.push_back(3);
+    if (!split_pow2(a, rmax, rad)) return false;
+    return plan_of_radices(n, rad, p, tw);
 }
 
 // Frequency bin held at position pos after the forward (decimation-in-frequency)
@@ -283,6 +290,8 @@ struct PassCfg {
     size_t smem = 0;  // one tile buffer (3 field regions)
     int grid = 0;     // CTAs of the single-instance kernel
     int line_nt = 0;  // t-pass: the line-specialised kernel's time axis (0: generic kernel)
+    int line_n = 0;   // x / y: the line-specialised body's axis length (0: generic kernel)
+    unsigned line_extent = 0;
     void *tw = nullptr;
     void *tab[2][3] = {};
     void *eom = nullptr;  // t-pass: EOM phase per time sample (natural order), or null
@@ -553,6 +562,38 @@ void default_variant(bool fp64, int kind, opo::PassVariant &v, size_t &te)
     te = fp64 ? 2048 : 4096;
 }
 
+// An x- or y-pass whose axis length has a compiled body (axis_line.cuh) runs it in place of
+// the generic tile, whatever classic CTA size, tile and radix the setting names: its plan
+// and geometry replace the generic ones.  The bodies measured faster than every generic
+// and warp-specialised variant at each compiled length.  They address a plane with 32-bit
+// byte offsets.
+template <typename C> void use_axis_line(const OpoParams &p, bool xa, PassCfg &pc, std::vector<cd> &tw)
+{
+    const int n = xa ? p.nx : p.ny;
+    if (!opo::axis_line_radix(xa, n, 0) || (size_t)p.nx * p.ny * sizeof(C) > 0xffffffffull) return;
+    std::vector<int> rad = {opo::axis_line_radix(xa, n, 0), opo::axis_line_radix(xa, n, 1)};
+    if (opo::axis_line_radix(xa, n, 2) > 1) rad.push_back(opo::axis_line_radix(xa, n, 2));
+    opo::AxisPlan plan;
+    std::vector<cd> t;
+    if (!plan_of_radices(n, rad, plan, t)) return;
+    pc.plan = plan;
+    tw = t;
+    pc.line_n = n;
+    const unsigned L = (unsigned)opo::axis_line_lines(sizeof(C) == 16, xa, n), nxy = (unsigned)p.nx * p.ny;
+    pc.line_extent = xa ? (unsigned)p.ny * p.nt : (unsigned)p.nx;
+    const unsigned per = (pc.line_extent + L - 1) / L;  // tiles of the field (x) or of one row (y)
+    opo::TileGeom &g = pc.geo;
+    g = opo::TileGeom{};
+    g.nlines = (int)L;
+    g.ntiles = (int)(xa ? per : per * (unsigned)p.nt);
+    g.tdiv = make_fastdiv(per);
+    g.tmulA = xa ? L * (unsigned)p.nx : L;
+    g.tmulB = xa ? 0u : nxy;
+    g.gs_j = xa ? 1u : (unsigned)p.nx;
+    g.gs_l = xa ? (unsigned)p.nx : 1u;
+    pc.smem = xa ? opo::axis_line_smem<C, true>(n) : opo::axis_line_smem<C, false>(n);
+}
+
 // Build the plan, geometry and tables of one pass kind for variant v and tile size te.
 template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVariant v, size_t te)
 {
@@ -699,8 +740,13 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
             }
         }
     }
+    if (kind != kT && !ws) use_axis_line<C>(s->p, kind == kX, pc, tw);
 
     int rc;
+    if (pc.line_n && pc.smem > 48 * 1024) {
+        cudaError_t e = kind == kX ? opo::configure_axis_line_t<C, true>(n) : opo::configure_axis_line_t<C, false>(n);
+        if (e != cudaSuccess) return cuda_fail(s, e, "configure line-specialised axis pass");
+    }
     if ((rc = upload<C>(s, pc.allocs, tw, &pc.tw))) { free_pass(pc); return rc; }
     const bool phys = (p.flags & OPO_PHYSICS) != 0;
     const opo::AxisPlan &pl = pc.plan;
@@ -708,6 +754,12 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
     const std::vector<double> comp = fp64 ? std::vector<double>() : opo::fp32_pair_compensation(pl, tw);
     auto fix = [&](std::vector<cd> &t) {
         if (!comp.empty()) opo::scale_table(t, comp);
+        if (pc.line_n && kind == kX) {  // the x bodies' table order (axis_line.cuh)
+            const std::vector<cd> pos = t;
+            const int rl = pl.radix[pl.ns - 1], ng = n / rl;
+            for (int g0 = 0; g0 < ng; g0++)
+                for (int k = 0; k < rl; k++) t[(size_t)k * ng + g0] = pos[(size_t)g0 * rl + k];
+        }
     };
     if (kind == kT) {
         // dispersion exp(i dz w (vinv + w b2/2)) exp(-alpha dz/2) / nt (Solver3D.cuh:153-169,
@@ -867,7 +919,9 @@ template <typename C> int configure_plane(OpoSolver *s, int K, int threads, int 
 // separate x and y passes when no cluster size fits the grid.
 template <typename C> int default_plane(OpoSolver *s)
 {
-    if (!(s->p.flags & OPO_DIFFRACTION)) return configure_plane<C>(s, 0, 256, 8);
+    // the line-specialised x and y passes measured faster than any plane pass
+    if (!(s->p.flags & OPO_DIFFRACTION) || (s->pass[kX].line_n && s->pass[kY].line_n))
+        return configure_plane<C>(s, 0, 256, 8);
     int chosen = 0;
     for (int K : {2, 4, 8}) {
         const size_t esz = sizeof(C);
@@ -949,6 +1003,8 @@ template <typename C> AxisArgs<C> make_axis_args(OpoSolver *s, int kind, int whi
     a.tw = static_cast<const C *>(pc.tw);
     for (int f = 0; f < 3; f++) a.tab[f] = tabs<C>(s, kind, which_tab)[f];
     a.tmask = mask;
+    a.line_n = pc.line_n;
+    a.line_extent = pc.line_extent;
     return a;
 }
 
@@ -992,6 +1048,11 @@ template <typename C> int enqueue_axis(OpoSolver *s, int kind, int which_tab, un
         OPO_CU(s, opo::launch_axis_ws<C>(a, w, pc.maps, opo::PassVariant{pc.v.threads - 32, pc.v.r1}, kind == kX,
                                          pc.grid, pc.smem, s->stream),
                "axis-pass launch");
+    } else if (pc.line_n) {
+        const bool square = s->p.nx == s->p.ny;
+        const cudaError_t e = kind == kX ? opo::launch_axis_line_t<C, true>(a, square, pc.smem, s->stream)
+                                         : opo::launch_axis_line_t<C, false>(a, square, pc.smem, s->stream);
+        OPO_CU(s, e, "axis-pass launch");
     } else {
         OPO_CU(s, opo::launch_axis<C>(a, pc.v, kind == kX, pc.grid, pc.smem, s->stream), "axis-pass launch");
     }
@@ -1267,6 +1328,18 @@ template <typename C> int autotune(OpoSolver *s)
         best.v[kind] = s->pass[kind].v;
         best.te[kind] = s->pass[kind].te;
         if (kind != kT && !(s->p.flags & OPO_DIFFRACTION)) continue;
+        if (kind != kT) {
+            // a compiled body runs whatever the classic setting: nothing to time
+            bool line = false;
+            for (int r1 : {8, 4})
+                if (!line && configure_pass<C>(s, kind, opo::PassVariant{128, r1}, tes[1]) == OPO_OK)
+                    line = s->pass[kind].line_n && s->pass[kind].v.r1 == r1;
+            if (line) {
+                best.v[kind] = s->pass[kind].v;
+                best.te[kind] = tes[1];
+                continue;
+            }
+        }
         for (size_t te : tes)
             for (int th : threads)
                 for (int r1 : r1s) {
@@ -1980,10 +2053,11 @@ bool solver_line_fallback_ok(const OpoSolver *s)
 }
 
 int solver_line_nt(const OpoSolver *s) { return s->pass[kT].line_nt; }
+int solver_line_n(const OpoSolver *s, int kind) { return s->pass[kind].line_n; }
 
 void solver_pass_info(const OpoSolver *s, int kind, int *ntiles, size_t *smem)
 {
-    *ntiles = s->pass[kind].geo.ntiles;
+    *ntiles = s->pass[kind].geo.ntiles * (s->pass[kind].line_n ? 3 : 1);  // a line tile holds one field
     *smem = s->pass[kind].smem;
 }
 

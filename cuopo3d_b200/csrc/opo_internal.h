@@ -100,6 +100,9 @@ template <typename C> struct AxisArgs {
     const C *tw;
     const typename TabOf<C>::type *tab[3];
     unsigned tmask;
+    int line_n;            // line-specialised body (axis_line.cuh): its axis length, else 0;
+                           // g then holds one field's tiles
+    unsigned line_extent;  // lines of a tile row (y: nx) or of the field (x: ny nt)
 };
 
 // Fused (x, y) diffraction pass over whole (field, t) planes.  A cluster of K CTAs owns
@@ -216,6 +219,15 @@ size_t tpass_line_smem(bool fp64, int nt, int r1);
 cudaError_t configure_line_kernels(size_t max_smem);
 template <typename C> cudaError_t launch_axis(const AxisArgs<C> &a, PassVariant v, bool bfast, int grid,
                                               size_t smem, cudaStream_t st);
+// Line-specialised axis pass (axis_line.cuh) of the fields in a.tmask; square: nx == ny (the
+// y-pass then compiles its row stride in).  configure_axis_line allows its kernels the full
+// shared memory.
+template <typename C, bool X>
+cudaError_t launch_axis_line_t(const AxisArgs<C> &a, bool square, size_t smem, cudaStream_t st);
+template <typename C, bool X> cudaError_t configure_axis_line_t(int n);
+// Batched form: the kernel over the line tiles of every instance, its CTA size in threads.
+struct BatchHeader;
+template <typename C, bool X> const void *axis_line_batch_func(int *threads);
 template <typename C> cudaError_t launch_sums(const C *f0, const C *f1, const C *f2, size_t n,
                                               double *partials, int nblocks, double *out,
                                               cudaStream_t st);

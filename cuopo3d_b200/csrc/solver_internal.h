@@ -27,6 +27,8 @@ PassVariant solver_pass_variant(const OpoSolver *s, int kind);
 bool solver_line_fallback_ok(const OpoSolver *s);
 // The line body's time axis the t-pass runs on s's grid (0: the generic body).
 int solver_line_nt(const OpoSolver *s);
+// The compiled axis length the x- or y-pass (kind 1, 2) runs on s's grid (0: the generic body).
+int solver_line_n(const OpoSolver *s, int kind);
 const OpoParams &solver_params(const OpoSolver *s);
 size_t solver_device_bytes(const OpoSolver *s);
 void *solver_field(OpoSolver *s, int which);

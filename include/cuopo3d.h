@@ -264,7 +264,10 @@ int opo_set_tuning(OpoSolver *s, const int tuning[9]);
  * bodies for the time axes 64, 128 and 256, tiles of 8 FP32 pixels (two per packed
  * instruction) or 4 FP64 pixels; other grids (and the shipped Q2 launch grid) run the
  * generic kernel of the same size with the fallback radix (FP32: the given radix, FP64:
- * 4).  No counterpart in the reference. */
+ * 4).  x- and y-passes whose axis length has a compiled body (16, 24, 32, 36, 48, 64, 72, 96,
+ * 108, 128, 144, 192, 216, 256, 384, 512) run it under every setting of 128 or 256 threads;
+ * such a setting's tile and radix then matter to other lengths only.  No counterpart in
+ * the reference. */
 #define OPO_TUNE_LINE 256
 int opo_get_tuning(const OpoSolver *s, int out[9]);
 
@@ -277,7 +280,7 @@ int opo_get_tuning(const OpoSolver *s, int out[9]);
  * both axes (4, 8 or 16; smaller when the plan needs it).  Fails with OPO_ERR_INVALID
  * when nx or ny is not a multiple of the cluster size or the slab does not fit; the
  * current configuration then stays.  Solvers start with a default plane pass where one
- * fits.  No counterpart in the reference (one cuFFT 3-D plan per field). */
+ * fits and the x or y length has no compiled body (opo_set_tuning).  No counterpart in the reference (one cuFFT 3-D plan per field). */
 int opo_set_plane_pass(OpoSolver *s, int cluster, int threads, int r1);
 /* {cluster size (0: separate x and y passes), threads, first-stage radix}. */
 int opo_get_plane_pass(const OpoSolver *s, int out[3]);
