@@ -22,7 +22,6 @@
 
 #include "batch_device.cuh"
 #include "pass_body.cuh"
-#include "tpass_line.cuh"
 #include "solver_internal.h"
 
 namespace opo {
@@ -53,35 +52,6 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 4 : 1)
         const C *src[3] = {d->psrc, d->f[1], d->f[2]};
         stage_tile<C, THREADS, false>(d->g, (unsigned)d->plan.n, tile, src, tpass_load_mask(*d), sm);
         tpass_tile<C, R1, THREADS, RMAX, true>(*d, tile, sm);
-    }
-}
-
-// Batched line-specialised t-pass for the instances whose time axis has the line body
-// (NT, RA): one tile at a time, one tile buffer.  Each line body has a kernel of its own
-// (one kernel holding every body and the generic one needed 168 registers and spilled);
-// the instances without a line body run tpass_batch_kernel with the fallback radix.
-template <typename C, int NT, int RA, int THREADS>
-__global__ void __launch_bounds__(THREADS, 4)
-    tpass_line_batch_kernel(const TPassArgs<C> *descs, const unsigned *prefix, const BatchHeader *hdr, int tp)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    TPassArgs<C> *d = reinterpret_cast<TPassArgs<C> *>(smem_raw);
-    unsigned char *buf = smem_raw + desc_bytes<TPassArgs<C>>();
-    const unsigned ninst = hdr->ninst, total = hdr->total_tiles;
-    descs += hdr->first;
-    prefix += hdr->pfirst;
-    int cur = -1;
-    for (unsigned gt = blockIdx.x; gt < total; gt += gridDim.x) {
-        const int i = find_inst(prefix, ninst, gt);
-        if (i != cur) {
-            __syncthreads();
-            stage_desc(descs + i, d);
-            __syncthreads();
-            if (threadIdx.x < 6 && d->ph_steps) d->ph[threadIdx.x / 3][threadIdx.x % 3] = d->ph_steps[tp * 6 + threadIdx.x];
-            __syncthreads();
-            cur = i;
-        }
-        tpass_line_tile<C, NT, RA, THREADS>(*d, gt - __ldg(prefix + i), buf);
     }
 }
 
@@ -170,14 +140,17 @@ __global__ void batch_tally_final_kernel(const double *partials, int nslots, dou
     X(float2, 256, 8, 16) X(float2, 256, 16, 16) X(double2, 128, 4, 8) X(double2, 128, 8, 8)        \
     X(double2, 256, 4, 16) X(double2, 256, 8, 16) X(double2, 256, 16, 16)
 
-// t-pass groups: under the line-specialised setting, the instances with the 256-, 128-
-// and 64-sample line bodies (groups 0-2) and the rest (group 3, the generic body with the
-// fallback radix); under any other setting every instance is in group 3.
-constexpr int kTGroups = 4;
-inline int t_group(PassVariant v, int line_nt)
+// t-pass groups: one per line body (tpass_line.cuh) -- the instances whose t-pass runs it --
+// and the rest (the generic body; under a line setting with its fallback radix).
+#define OPO_ITEM(NT) NT,
+constexpr int kLineNT[] = {OPO_TPASS_LINE_SETTINGS(OPO_ITEM) OPO_TPASS_LINES(OPO_ITEM)};
+#undef OPO_ITEM
+constexpr int kTGroups = (int)(sizeof(kLineNT) / sizeof(kLineNT[0])) + 1;
+inline int t_group(int line_nt)
 {
-    if (!is_line(v)) return 3;
-    return line_nt == 256 ? 0 : line_nt == 128 ? 1 : line_nt == 64 ? 2 : 3;
+    for (int g = 0; g < kTGroups - 1; g++)
+        if (kLineNT[g] == line_nt) return g;
+    return kTGroups - 1;
 }
 
 // x and y groups: the instances whose axis length has a compiled body (axis_line.cuh; one
@@ -186,17 +159,18 @@ constexpr int kAxGroups = 2;
 
 template <typename C> bool batch_t_generic_func(PassVariant v, const void **fn);
 
-// Resolves the batched kernel of each t-pass group (nullptr: the group is never
-// populated under this setting); returns false if a variant is not compiled.
-template <typename C> bool batch_t_funcs(PassVariant v, const void *fn[kTGroups])
+// Resolves the batched kernel and CTA size of each t-pass group; returns false if a variant
+// is not compiled.
+template <typename C> bool batch_t_funcs(PassVariant v, const void *fn[kTGroups], int threads[kTGroups])
 {
-    for (int g = 0; g < kTGroups; g++) fn[g] = nullptr;
-    if (!is_line(v)) return batch_t_generic_func<C>(v, &fn[3]);
-    if (v.threads != 128 || !line_variant_compiled(v.threads, radix_of(v))) return false;
-    fn[0] = reinterpret_cast<const void *>(tpass_line_batch_kernel<C, 256, 16, 128>);
-    fn[1] = reinterpret_cast<const void *>(tpass_line_batch_kernel<C, 128, 16, 128>);
-    fn[2] = reinterpret_cast<const void *>(tpass_line_batch_kernel<C, 64, 8, 128>);
-    return batch_t_generic_func<C>(PassVariant{128, line_fallback_radix(sizeof(C) == 16, v)}, &fn[3]);
+    for (int g = 0; g < kTGroups - 1; g++) {
+        fn[g] = tpass_line_batch_func<C>(kLineNT[g]);
+        threads[g] = tpass_line_shape(kLineNT[g]).threads;
+    }
+    threads[kTGroups - 1] = v.threads;
+    if (!is_line(v)) return batch_t_generic_func<C>(v, &fn[kTGroups - 1]);
+    if (!line_variant_compiled(v.threads, radix_of(v))) return false;
+    return batch_t_generic_func<C>(PassVariant{128, line_fallback_radix(sizeof(C) == 16, v)}, &fn[kTGroups - 1]);
 }
 
 template <typename C> bool batch_t_generic_func(PassVariant v, const void **fn)
@@ -341,7 +315,7 @@ template <typename C> int upload_descriptors(OpoBatch *b)
             ax[a][0].push_back(opo::make_axis_args<C>(s, 1 + a, 0, diff ? 7u : 0u));
             ax[a][1].push_back(opo::make_axis_args<C>(s, 1 + a, 1, (diff && !last) ? 6u : 0u));
         }
-        tgroup.push_back(opo::t_group(b->v[0], opo::solver_line_nt(s)));
+        tgroup.push_back(opo::t_group(opo::solver_line_nt(s)));
         opo::SlotFields f;
         for (int k = 0; k < 3; k++) f.f[k] = opo::solver_field(s, k + 1);
         f.n = (unsigned long long)sl.voxels;
@@ -420,13 +394,14 @@ int persistent_grid(OpoBatch *b, const void *fn, int threads, size_t smem)
 // Kernels of every group: t-pass groups, and per axis the line bodies and the generic body.
 template <typename C> struct BatchFuncs {
     const void *t[opo::kTGroups];
+    int t_threads[opo::kTGroups];
     const void *ax[2][opo::kAxGroups];
     int ax_threads[2][opo::kAxGroups];
 };
 
 template <typename C> bool batch_funcs(const OpoBatch *b, BatchFuncs<C> &f)
 {
-    if (!opo::batch_t_funcs<C>(b->v[0], f.t) || !opo::batch_a_func<C>(b->v[1], true, &f.ax[0][1]) ||
+    if (!opo::batch_t_funcs<C>(b->v[0], f.t, f.t_threads) || !opo::batch_a_func<C>(b->v[1], true, &f.ax[0][1]) ||
         !opo::batch_a_func<C>(b->v[2], false, &f.ax[1][1]))
         return false;
     f.ax[0][0] = opo::axis_line_batch_func<C, true>(&f.ax_threads[0][0]);
@@ -452,7 +427,7 @@ template <typename C> int enqueue_batch_round_trip(OpoBatch *b)
             const opo::BatchHeader *h = hdr + g;
             void *args[] = {(void *)&descs, (void *)&pre, (void *)&h, (void *)&tp};
             b->launches++;
-            cudaError_t e = cudaLaunchKernel(f.t[g], dim3(b->t_group[g].grid), dim3(b->v[0].threads), args,
+            cudaError_t e = cudaLaunchKernel(f.t[g], dim3(b->t_group[g].grid), dim3(f.t_threads[g]), args,
                                              b->t_group[g].smem, b->stream);
             if (e != cudaSuccess) return e;
         }
@@ -505,7 +480,7 @@ bool graph_covers(OpoBatch *b, bool grow)
                                                    : opo::desc_bytes<opo::TPassArgs<float2>>();
         const size_t da = b->precision == OPO_FP64 ? opo::desc_bytes<opo::AxisArgs<double2>>()
                                                    : opo::desc_bytes<opo::AxisArgs<float2>>();
-        need(b->t_group[opo::t_group(b->v[0], opo::solver_line_nt(s))], dt + sm);
+        need(b->t_group[opo::t_group(opo::solver_line_nt(s))], dt + sm);
         for (int a = 0; a < 2; a++) {
             opo::solver_pass_info(s, 1 + a, &nt, &sm);
             need(b->ax_group[a][ax_group_of(s, 1 + a)], da + sm);
@@ -531,7 +506,7 @@ template <typename C> int build_batch_graph(OpoBatch *b)
         return OPO_OK;
     };
     for (int g = 0; g < opo::kTGroups; g++)
-        if (int rc = configure(b->t_group[g], f.t[g], b->v[0].threads)) return rc;
+        if (int rc = configure(b->t_group[g], f.t[g], f.t_threads[g])) return rc;
     for (int a = 0; a < 2; a++)
         for (int g = 0; g < opo::kAxGroups; g++)
             if (int rc = configure(b->ax_group[a][g], f.ax[a][g], f.ax_threads[a][g])) return rc;
@@ -625,7 +600,8 @@ int opo_batch_create(int precision, int capacity, size_t hbm_budget, const int t
             b->v[k] = opo::PassVariant{opo::consumer_threads(opo::PassVariant{tuning[3 * k], 0}), tuning[3 * k + 2]};
             b->te[k] = (size_t)tuning[3 * k + 1];
         } else {
-            b->v[k] = opo::PassVariant{128, k == 0 ? 4 : 8};
+            // t: the line bodies where a grid has one, else radix 4
+            b->v[k] = opo::PassVariant{128, k == 0 ? opo::kLineForm | 4 : 8};
             b->te[k] = fp64 ? 1024 : 2048;
         }
         if (!opo::variant_compiled(fp64, k == 0, b->v[k])) {

@@ -553,10 +553,21 @@ void diffraction_tables(const OpoParams &p, bool xa, const opo::AxisPlan &pl, st
     }
 }
 
-// Default variant and tile size of a pass kind: 96 KB of shared memory for the three
-// fields (4096 complex64 or 2048 complex128 per field), 256 threads.
-void default_variant(bool fp64, int kind, opo::PassVariant &v, size_t &te)
+template <typename C> bool tpass_line_body(const OpoParams &p, opo::PassVariant v);
+
+// Default variant and tile size of a pass kind: the line t-pass where the grid has a body
+// (128 x 128 x 256: FP32 70 against 105 us, FP64 124 against 223 us), otherwise 96 KB of
+// shared memory for the three fields (4096 complex64 or 2048 complex128 per field), 256
+// threads.
+void default_variant(const OpoParams &p, int kind, opo::PassVariant &v, size_t &te)
 {
+    const bool fp64 = p.precision == OPO_FP64;
+    const opo::PassVariant line{128, opo::kLineForm | (fp64 ? 4 : 16)};
+    if (kind == kT && (fp64 ? tpass_line_body<double2>(p, line) : tpass_line_body<float2>(p, line))) {
+        v = line;
+        te = fp64 ? 1024 : 2048;
+        return;
+    }
     v.threads = 256;
     v.r1 = (fp64 && kind == kT) ? 8 : 16;
     te = fp64 ? 2048 : 4096;
@@ -594,6 +605,35 @@ template <typename C> void use_axis_line(const OpoParams &p, bool xa, PassCfg &p
     pc.smem = xa ? opo::axis_line_smem<C, true>(n) : opo::axis_line_smem<C, false>(n);
 }
 
+// Whether the t-pass of setting v runs a line body on this grid.
+template <typename C> bool tpass_line_body(const OpoParams &p, opo::PassVariant v)
+{
+    const bool fp64 = sizeof(C) == 16;
+    const opo::LineShape sh = opo::tpass_line_shape(p.nt);
+    if (opo::is_ws(v) || (p.flags & OPO_ASIS_Q2) || !sh.ra) return false;
+    if ((size_t)p.nx * p.ny % (sh.pp * (fp64 ? 1 : 2))) return false;  // whole tiles only
+    return !opo::line_setting_only(p.nt) || (opo::is_line(v) && p.nx % opo::line_pixels(fp64) == 0);
+}
+
+// The line body's plan and geometry in place of the generic ones.
+template <typename C> bool use_tpass_line(const OpoParams &p, PassCfg &pc, std::vector<cd> &tw)
+{
+    const opo::LineShape sh = opo::tpass_line_shape(p.nt);
+    std::vector<int> rad = {sh.ra, sh.rb};
+    if (sh.rc > 1) rad.push_back(sh.rc);
+    if (!plan_of_radices(p.nt, rad, pc.plan, tw)) return false;
+    const unsigned P = (unsigned)sh.pp * (sizeof(C) == 16 ? 1 : 2), nxy = (unsigned)p.nx * p.ny;
+    opo::TileGeom &g = pc.geo;
+    g = opo::TileGeom{};
+    g.nlines = (int)P;
+    g.ntiles = (int)(nxy / P);
+    g.gs_j = nxy;
+    g.gs_l = 1;
+    pc.line_nt = p.nt;
+    pc.smem = opo::tpass_line_smem<C>(p.nt);
+    return true;
+}
+
 // Build the plan, geometry and tables of one pass kind for variant v and tile size te.
 template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVariant v, size_t te)
 {
@@ -619,29 +659,20 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
     std::vector<cd> tw;
     const int form = v.r1 & opo::kLineForm;
     int r1 = opo::radix_of(v);
-    // line-specialised t-pass: a compiled time axis with its two-stage plan, whole tiles of
-    // line_pixels() pixels, and every pixel transformed (not the shipped Q2 launch grid);
-    // otherwise its generic fallback radix
-    const int LP = opo::line_pixels(fp64);
-    const bool line = form && kind == kT && opo::line_radix(nt) && nx % LP == 0 && !(p.flags & OPO_ASIS_Q2);
-    if (line) r1 = opo::line_radix(nt);
-    else if (form) r1 = opo::line_fallback_radix(fp64, v);
+    // line-specialised t-pass (tpass_line.cuh): every pixel transformed (not the shipped Q2
+    // launch grid), and for a line setting's own axes nx a multiple of its tile; otherwise
+    // a line setting's generic fallback radix
+    const bool line = kind == kT && tpass_line_body<C>(p, v);
+    if (form) r1 = opo::line_fallback_radix(fp64, v);
     else if (fp64 && kind == kT) r1 = std::min(r1, 8);  // 3 fields x r1 complex128 live in registers
-    while (r1 >= 4 && !build_plan(n, r1, line ? 16 : opo::variant_max_radix(fp64, v), pc.plan, tw)) r1 /= 2;
+    while (r1 >= 4 && !build_plan(n, r1, opo::variant_max_radix(fp64, v), pc.plan, tw)) r1 /= 2;
     if (r1 < 4) return fail(s, OPO_ERR_INVALID, "grid sizes must be 2^a 3^b and >= 8");
     // a line variant keeps its setting (the bodies fix their radices); the fallback's
     // radix is checked by batches (solver_line_fallback_ok)
     pc.v.r1 = form ? v.r1 : r1;
-    if (line && pc.plan.ns == 2) pc.line_nt = nt;
     const unsigned nxy = (unsigned)nx * ny;
     opo::TileGeom &g = pc.geo;
-    if (pc.line_nt) {
-        pc.te = (size_t)nt * LP;
-        g.nlines = LP; g.ntiles = (nx / LP) * ny;
-        g.lsl = 1; g.lsj = LP; g.region = (unsigned)(nt * LP);  // (the kernels lay out their own tiles)
-        g.tdiv = make_fastdiv(nx / LP); g.tmulA = LP; g.tmulB = nx; g.gs_j = nxy; g.gs_l = 1;
-        g.pairs = 1;
-    } else if (kind == kT) {
+    if (kind == kT) {
         const int P = largest_divisor_leq(nx, (int)(te / nt));
         g.nlines = P; g.ntiles = (nx / P) * ny;
         g.lsl = 1; g.lsj = P; g.region = (unsigned)(nt * P);
@@ -663,7 +694,7 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
         g.tdiv = make_fastdiv(1); g.tmulA = 0; g.tmulB = (unsigned)rows * nx; g.gs_j = 1; g.gs_l = nx;
     }
     const bool ws = opo::is_ws(v);
-    if (kind != kX && !ws && !pc.line_nt && g.lsj * sizeof(C) < (fp64 ? 128u : 64u)) {
+    if (kind != kX && !ws && g.lsj * sizeof(C) < (fp64 ? 128u : 64u)) {
         // Line groups narrower than a shared-memory wavefront: the last forward stage's
         // butterflies (R rows apart, R its radix) would all fall on the same banks, so
         // one padding row follows every R rows.  Every earlier stage has a stride that
@@ -688,8 +719,8 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
         const unsigned per128 = (unsigned)(128 / sizeof(C));
         g.region = (g.region + per128 - 1) / per128 * per128;
     }
-    pc.smem = pc.line_nt ? opo::tpass_line_smem(fp64, nt, r1) : 3 * (size_t)g.region * sizeof(C);
-    if (pc.smem > 227 * 1024) return fail(s, OPO_ERR_INVALID, "tile does not fit in shared memory");
+    pc.smem = 3 * (size_t)g.region * sizeof(C);
+    if (pc.smem > 227 * 1024 && !(line && form)) return fail(s, OPO_ERR_INVALID, "tile does not fit in shared memory");
     if (ws) {
         opo::WsArgs &w = pc.wsa;
         const size_t es = sizeof(C);
@@ -741,8 +772,16 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
         }
     }
     if (kind != kT && !ws) use_axis_line<C>(s->p, kind == kX, pc, tw);
+    if (line) {
+        if (!use_tpass_line<C>(p, pc, tw)) return fail(s, OPO_ERR_INVALID, "line-specialised t-pass plan");
+        if (form) pc.te = (size_t)nt * opo::line_pixels(fp64);
+    }
 
     int rc;
+    if (pc.line_nt && pc.smem > 48 * 1024) {
+        cudaError_t e = opo::configure_line_kernels<C>(nt, 227 * 1024);
+        if (e != cudaSuccess) return cuda_fail(s, e, "configure line-specialised t-pass");
+    }
     if (pc.line_n && pc.smem > 48 * 1024) {
         cudaError_t e = kind == kX ? opo::configure_axis_line_t<C, true>(n) : opo::configure_axis_line_t<C, false>(n);
         if (e != cudaSuccess) return cuda_fail(s, e, "configure line-specialised axis pass");
@@ -1025,8 +1064,10 @@ int enqueue_t(OpoSolver *s, bool reset_pump, int n_rk4, const double *zh, int wh
         OPO_CU(s, opo::launch_tpass_ws<C>(a, w, maps, opo::PassVariant{pc.v.threads - 32, pc.v.r1}, pc.grid, pc.smem,
                                           s->stream),
                "t-pass launch");
+    } else if (pc.line_nt) {
+        OPO_CU(s, opo::launch_tpass_line<C>(a, pc.line_nt, pc.grid, pc.smem, s->stream), "t-pass launch");
     } else if (opo::is_line(pc.v)) {
-        OPO_CU(s, opo::launch_tpass_line<C>(a, pc.v, pc.line_nt, pc.plan.radix[0], pc.grid, pc.smem, s->stream),
+        OPO_CU(s, opo::launch_tpass_line_fallback<C>(a, pc.v, pc.plan.radix[0], pc.grid, pc.smem, s->stream),
                "t-pass launch");
     } else {
         OPO_CU(s, opo::launch_tpass<C>(a, opo::PassVariant{pc.v.threads, opo::radix_of(pc.v)}, pc.grid, pc.smem,
@@ -1328,12 +1369,12 @@ template <typename C> int autotune(OpoSolver *s)
         best.v[kind] = s->pass[kind].v;
         best.te[kind] = s->pass[kind].te;
         if (kind != kT && !(s->p.flags & OPO_DIFFRACTION)) continue;
-        if (kind != kT) {
-            // a compiled body runs whatever the classic setting: nothing to time
+        {
+            // a body that runs whatever the classic setting: nothing to time
             bool line = false;
             for (int r1 : {8, 4})
                 if (!line && configure_pass<C>(s, kind, opo::PassVariant{128, r1}, tes[1]) == OPO_OK)
-                    line = s->pass[kind].line_n && s->pass[kind].v.r1 == r1;
+                    line = (s->pass[kind].line_n || s->pass[kind].line_nt) && s->pass[kind].v.r1 == r1;
             if (line) {
                 best.v[kind] = s->pass[kind].v;
                 best.te[kind] = tes[1];
@@ -1355,7 +1396,7 @@ template <typename C> int autotune(OpoSolver *s)
                         best.te[kind] = te;
                     }
                 }
-        // line-specialised FP32 t-pass variants, where the grid has a compiled form
+        // the line setting, where the grid has a body that only it runs
         for (int r1 : r1s) {
             const opo::PassVariant lv{128, r1 | opo::kLineForm};
             // one candidate per precision: its fallback radix (FP32 16, FP64 4) only matters
@@ -1659,14 +1700,15 @@ static int create_impl(const OpoParams *p, const double *w, const opo::PassVaria
         if ((e = opo::configure_kernels(227 * 1024)) != cudaSuccess ||
             (e = opo::configure_plane_kernels(227 * 1024)) != cudaSuccess ||
             (e = opo::configure_ws_kernels(227 * 1024)) != cudaSuccess ||
-            (e = opo::configure_line_kernels(227 * 1024)) != cudaSuccess) {
+            (e = opo::configure_line_kernels<float2>(0, 227 * 1024)) != cudaSuccess ||
+            (e = opo::configure_line_kernels<double2>(0, 227 * 1024)) != cudaSuccess) {
             rc = cuda_fail(s, e, "configure kernels");
             break;
         }
         for (int k = 0; k < 3 && !rc; k++) {
             opo::PassVariant v;
             size_t te;
-            default_variant(p->precision == OPO_FP64, k, v, te);
+            default_variant(s->p, k, v, te);
             if (vv && tt) {
                 v = vv[k];
                 te = tt[k];

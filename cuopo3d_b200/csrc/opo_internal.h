@@ -90,7 +90,7 @@ template <typename C> struct TPassArgs {
     unsigned nx;        // grid width (for the row test above)
     const C *eom;       // per time sample: exp(i beta sin(2 pi fpm t)) on signal and idler
                         // after the half steps (closing pass of a round trip), or null
-    int line_nt;        // line-specialised FP32 form (tpass_line.cuh): its time axis, else 0
+    int line_nt;        // line-specialised form (tpass_line.cuh): its time axis, else 0
 };
 
 template <typename C> struct AxisArgs {
@@ -161,21 +161,58 @@ struct PassVariant {
 };
 
 // Flag in PassVariant::r1 (and in the r1 entries of the C-ABI tuning arrays): the
-// line-specialised t-pass (tpass_line.cuh: tiles of 8 FP32 or 4 FP64 pixels, FP32
-// split-pair arithmetic) on CTAs of 128 threads, for every time axis with a compiled
-// body (64, 128, 256; the body fixes its own radices).  Grids it does not cover (another
-// time axis, nx not a multiple of the tile, the shipped Q2 launch grid) run the generic
-// tile body at the same CTA size with the fallback radix: the variant's radix in FP32,
-// radix 4 (the register form) in FP64.
+// line-specialised t-pass (tpass_line.cuh: FP32 split-pair arithmetic, compile-time plans)
+// also for the time axes 64, 128 and 256 where nx is a multiple of line_pixels(); other
+// axes with a line body run it under every setting.  Grids without one (another time axis,
+// the shipped Q2 launch grid) run the generic tile body at the setting's CTA size (128)
+// with the fallback radix: the variant's radix in FP32, radix 4 (the register form) in
+// FP64.
 constexpr int kLineForm = 256;
-inline int line_pixels(bool fp64) { return fp64 ? 4 : 8; }  // pixels per tile
+inline int line_pixels(bool fp64) { return fp64 ? 4 : 8; }  // nx multiple of a line setting
 inline bool is_line(PassVariant v) { return (v.r1 & kLineForm) != 0; }
 inline int radix_of(PassVariant v) { return v.r1 & (kLineForm - 1); }
 // Line-specialised t-pass kernels: CTA size and the radix of the generic fallback.
 inline bool line_variant_compiled(int threads, int r1) { return threads == 128 && (r1 == 4 || r1 == 8 || r1 == 16); }
 inline int line_fallback_radix(bool fp64, PassVariant v) { return fp64 ? 4 : radix_of(v); }
-// First-stage radix of the compiled line body for a time axis of n samples (0: none).
-inline int line_radix(int n) { return (n == 256 || n == 128) ? 16 : (n == 64 ? 8 : 0); }
+// Compiled line bodies by time axis: X(NT).  The first three run under a line setting only;
+// the others replace the generic tile bodies under every setting of 128 or 256 threads (the
+// generic forms took 1.3-1.9 times as long on their lengths).
+#define OPO_TPASS_LINE_SETTINGS(X) X(64) X(128) X(256)
+#define OPO_TPASS_LINES(X)                                                                         \
+    X(32) X(36) X(48) X(72) X(96) X(108) X(144) X(192) X(216) X(288) X(384) X(432) X(512) X(576)    \
+    X(768) X(864) X(1024)
+// Radices (rc = 1: two stages), 16-byte units per time sample, CTA size and CTAs per SM of a
+// line body (tpass_line.cuh); ra = 0: none.
+struct LineShape {
+    int ra, rb, rc, pp, threads, ctas;
+};
+__host__ __device__ constexpr LineShape tpass_line_shape(int nt)
+{
+    switch (nt) {
+    case 32: return {8, 4, 1, 8, 64, 8};
+    case 36: return {6, 6, 1, 8, 64, 8};
+    case 48: return {6, 8, 1, 8, 128, 4};
+    case 64: return {8, 8, 1, 8, 128, 4};
+    case 72: return {9, 8, 1, 8, 192, 3};
+    case 96: return {12, 8, 1, 8, 128, 4};
+    case 108: return {9, 12, 1, 8, 192, 3};
+    case 128: return {16, 8, 1, 8, 128, 4};
+    case 144: return {12, 12, 1, 8, 192, 3};
+    case 192: return {16, 12, 1, 4, 128, 4};
+    case 216: return {9, 6, 4, 4, 192, 3};
+    case 256: return {16, 16, 1, 4, 128, 4};
+    case 288: return {6, 6, 8, 4, 192, 3};
+    case 384: return {8, 6, 8, 4, 256, 2};
+    case 432: return {9, 6, 8, 4, 256, 2};
+    case 512: return {8, 8, 8, 4, 256, 2};
+    case 576: return {9, 8, 8, 2, 192, 3};
+    case 768: return {12, 8, 8, 2, 256, 2};
+    case 864: return {12, 9, 8, 2, 256, 2};
+    case 1024: return {16, 8, 8, 2, 256, 2};
+    default: return {0, 0, 0, 0, 0, 0};
+    }
+}
+inline bool line_setting_only(int nt) { return nt == 64 || nt == 128 || nt == 256; }
 // Largest radix of the generic fallback body at a line variant's CTA size.
 template <typename C, int THREADS> struct LineFallback {
     static constexpr int RMAX = (sizeof(C) == 16 && THREADS == 128) ? 8 : 16;
@@ -208,15 +245,20 @@ inline bool variant_compiled(bool fp64, bool tpass, PassVariant v)
 // cudaErrorInvalidValue for a variant that is not compiled.
 template <typename C> cudaError_t launch_tpass(const TPassArgs<C> &a, PassVariant v, int grid, size_t smem,
                                                cudaStream_t st);
-// Line-specialised t-pass (v.r1 carries kLineForm) for a time axis of nt samples; nt = 0:
-// the generic tile body at the variant's CTA size with first-stage radix r_fallback
-// (the plan's).
+// Line-specialised t-pass for a time axis with a line body.
+template <typename C> cudaError_t launch_tpass_line(const TPassArgs<C> &a, int nt, int grid, size_t smem, cudaStream_t st);
+// The generic tile body a line setting falls back to: its CTA size with first-stage radix
+// r_fallback (the plan's).
 template <typename C>
-cudaError_t launch_tpass_line(const TPassArgs<C> &a, PassVariant v, int nt, int r_fallback, int grid, size_t smem,
-                              cudaStream_t st);
-// Dynamic shared memory of a line-specialised t-pass CTA (0: nt / r1 not compiled).
-size_t tpass_line_smem(bool fp64, int nt, int r1);
-cudaError_t configure_line_kernels(size_t max_smem);
+cudaError_t launch_tpass_line_fallback(const TPassArgs<C> &a, PassVariant v, int r_fallback, int grid, size_t smem,
+                                       cudaStream_t st);
+// Dynamic shared memory of a line-specialised t-pass CTA.
+template <typename C> size_t tpass_line_smem(int nt);
+// Allows the line kernels of nt (and, with nt = 0, the fallback kernels) the full shared memory.
+template <typename C> cudaError_t configure_line_kernels(int nt, size_t max_smem);
+// The batched kernel of line body nt.
+struct BatchHeader;
+template <typename C> const void *tpass_line_batch_func(int nt);
 template <typename C> cudaError_t launch_axis(const AxisArgs<C> &a, PassVariant v, bool bfast, int grid,
                                               size_t smem, cudaStream_t st);
 // Line-specialised axis pass (axis_line.cuh) of the fields in a.tmask; square: nx == ny (the
@@ -226,7 +268,6 @@ template <typename C, bool X>
 cudaError_t launch_axis_line_t(const AxisArgs<C> &a, bool square, size_t smem, cudaStream_t st);
 template <typename C, bool X> cudaError_t configure_axis_line_t(int n);
 // Batched form: the kernel over the line tiles of every instance, its CTA size in threads.
-struct BatchHeader;
 template <typename C, bool X> const void *axis_line_batch_func(int *threads);
 template <typename C> cudaError_t launch_sums(const C *f0, const C *f1, const C *f2, size_t n,
                                               double *partials, int nblocks, double *out,

@@ -1,30 +1,33 @@
 // Line-specialised t-pass: the tile body of tpass_tile / tpass_tile_split for a time
-// axis whose length and radix plan are compile-time constants (NT = RA x RB with RA, RB
-// in {8, 16}: 64, 128, 256), in FP32 and FP64.
+// axis whose length and radix plan are compile-time constants, in FP32 and FP64.
 //
 // It computes what the generic t-pass computes (reference Solver3D.cuh:872-943 RK4 half
 // steps, then Solver3D.cuh:572-639 dispersion: transform, phase, inverse transform) on
-// tiles of 16-byte units: four units per time sample, one time sample per shared-memory
+// tiles of 16-byte units: PP units per time sample, one time sample per shared-memory
 // row.  A unit is one FP64 pixel, or in FP32 a split pair: the same time sample of
 // pixels l and l + 1, real parts in one packed f32x2 register pair and imaginary parts
 // in another, in registers and in shared memory (re_l, re_l+1, im_l, im_l+1).  Every FP32
 // butterfly, twiddle and phase product then serves two lines with one packed instruction
 // per component (a complex product: 4 packed instructions for two values; multiplying by
 // +-i only renames registers), each twiddle and phase factor is loaded once for both
-// lines, and all index arithmetic is compile-time.  A tile is 8 pixels (FP32) or 4
-// (FP64) of one row.  The transforms are the generic two-stage plan [RA, RB] (decimation
-// in frequency forward, in time inverse, phase tables in the plan's digit-reversed
-// order), so the twiddles and phase tables are the host's tables of that plan.
+// lines, and all index arithmetic is compile-time.  The pixels of a tile are consecutive in
+// the (x, y) plane, whatever nx; the plane holds whole tiles.  The transforms are two-stage plans [RA, RB] up to 256
+// samples and three-stage plans [RA, RB, RC] beyond (decimation in frequency forward, in
+// time inverse, phase tables in the plan's digit-reversed order), so the twiddles and
+// phase tables are the host's tables of that plan.
 //
-// Shared memory per field: NT + NT / RB rows of four units; time sample t sits in row
-// t + t / RB (a padding row after every RB rows), so the RB-point stage's eight
-// butterflies of a warp fall on alternating halves of the banks, and the other stages
-// read whole 512-byte runs.  The first stage's twiddles are staged with the tile, after
-// the three field regions (shared-memory latency instead of L1 for the 30 twiddle loads
-// of a first- and last-stage item; the phase tables stay in global memory).
+// Shapes (tpass_line_shape): PP and the CTA size give each stage about one item per thread of
+// half a CTA (two (stage, field) jobs run at a time) and 12-18 warps per SM beside tiles
+// of 20-110 KB.  The pass is bound by its arithmetic pipes and by latency (128 x 128 x 256:
+// FP32 FMA pipe 61 %, FP64 pipe 65 % busy), so warps per SM and whole warps per stage decide.
 //
-// The single-instance kernel runs one tile per CTA, four CTAs of 128 threads per SM; the
-// batched kernel runs the same body over the tiles of every instance.
+// Shared memory per field: NT rows of PP units.  With PP < 8 the last stage's threads, RL
+// rows apart, would share banks: two-stage bodies put a padding row after every RL rows,
+// three-stage ones (whose tiles leave no room) put time sample t in row t ^ (t / RL mod 8 / PP),
+// a permutation inside each group of RL rows (at 256 samples the permutation's index
+// arithmetic cost 4 %: FP32 73.7 against 70.7 us).  The first stage's twiddles are staged with
+// the tile, after the three field regions (shared-memory latency instead of L1 for the
+// twiddle loads of a first- and last-stage item; the other tables stay in global memory).
 #pragma once
 
 #include "pass_body.cuh"
@@ -116,6 +119,85 @@ template <int S, bool ROT2 = false> __device__ __forceinline__ void xdft4(X2C &x
 }
 
 template <int R, int S> struct XDft;
+
+template <int S> struct XDft<2, S> {
+    __device__ __forceinline__ static void run(X2C *x)
+    {
+        const X2C t = x[0];
+        x[0] = xadd(t, x[1]);
+        x[1] = xsub(t, x[1]);
+    }
+};
+
+template <int S> struct XDft<3, S> {
+    __device__ __forceinline__ static void run(X2C *x)
+    {
+        const f32x2 h = x2_dup(-0.5f), s3 = x2_dup(S * Roots<float>::s3), n3 = x2_dup(-S * Roots<float>::s3);
+        const X2C t = xadd(x[1], x[2]), d = xsub(x[1], x[2]);
+        const X2C m{xr_fma(t.r, h, x[0].r), xr_fma(t.i, h, x[0].i)};
+        x[0] = xadd(x[0], t);
+        x[1] = X2C{xr_fma(d.i, n3, m.r), xr_fma(d.r, s3, m.i)};  // m + S i s3 d
+        x[2] = X2C{xr_fma(d.i, s3, m.r), xr_fma(d.r, n3, m.i)};
+    }
+};
+
+template <int S> struct XDft<4, S> {
+    __device__ __forceinline__ static void run(X2C *x) { xdft4<S>(x[0], x[1], x[2], x[3]); }
+};
+
+// 6 = 2 x 3 and 12 = 4 x 3 by the prime-factor map (dft_3xm)
+template <int M, int S> __device__ __forceinline__ void xdft_3xm(X2C *x)
+{
+    constexpr int N = 3 * M, E = M == 4 ? 9 : 3;
+    X2C y[N];
+#pragma unroll
+    for (int n2 = 0; n2 < M; n2++) {
+        X2C t[3] = {x[3 * n2 % N], x[(M + 3 * n2) % N], x[(2 * M + 3 * n2) % N]};
+        XDft<3, S>::run(t);
+        y[n2] = t[0];
+        y[M + n2] = t[1];
+        y[2 * M + n2] = t[2];
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < 3; k1++) {
+        XDft<M, S>::run(y + M * k1);
+#pragma unroll
+        for (int k2 = 0; k2 < M; k2++) x[(4 * k1 + E * k2) % N] = y[M * k1 + k2];
+    }
+}
+template <int S> struct XDft<6, S> {
+    __device__ __forceinline__ static void run(X2C *x) { xdft_3xm<2, S>(x); }
+};
+template <int S> struct XDft<12, S> {
+    __device__ __forceinline__ static void run(X2C *x) { xdft_3xm<4, S>(x); }
+};
+
+// 9 = 3 x 3 as Dft<9>
+template <int S> struct XDft<9, S> {
+    __device__ __forceinline__ static void run(X2C *x)
+    {
+        using K = Roots<float>;
+        X2C u[3][3];
+#pragma unroll
+        for (int m = 0; m < 3; m++) {
+            X2C t[3] = {x[m], x[m + 3], x[m + 6]};
+            XDft<3, S>::run(t);
+            u[0][m] = t[0];
+            u[1][m] = t[1];
+            u[2][m] = t[2];
+        }
+        u[1][1] = xrot<S>(u[1][1], K::c9, K::s9);
+        u[1][2] = xrot<S>(u[1][2], K::c9_2, K::s9_2);
+        u[2][1] = xrot<S>(u[2][1], K::c9_2, K::s9_2);
+        u[2][2] = xrot<S>(u[2][2], K::c9_4, K::s9_4);
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            XDft<3, S>::run(u[r]);
+#pragma unroll
+            for (int k = 0; k < 3; k++) x[3 * k + r] = u[r][k];
+        }
+    }
+};
 
 // 8 = 2 x 4: a_m = x_m + x_{m+4}, b_m = (x_m - x_{m+4}) W8^m, y_{2k} = DFT4(a), y_{2k+1} = DFT4(b)
 template <int S> struct XDft<8, S> {
@@ -242,37 +324,44 @@ template <> struct LineUnit<double2> {
     }
 };
 
-template <typename C, int NT, int RA> struct LineGeom {
-    static constexpr int RB = NT / RA;
-    static constexpr int Q = RB;  // butterflies per line of the RA-point stage
-    static constexpr int PP = 4;  // units per row (time sample)
-    static constexpr int P = PP * LineUnit<C>::PX;  // pixels per tile
-    static constexpr int ROWS = NT + NT / RB;
-    static constexpr int REGION = ROWS * PP * 16;  // bytes per field region
-    static constexpr int A = PP * Q;   // RA-point butterflies per field
-    static constexpr int B = PP * RA;  // RB-point butterflies per field
-    __device__ __forceinline__ static constexpr int row(int t) { return t + t / RB; }
-    // byte offset of (field f, time sample t, unit u) in a tile buffer
-    __device__ __forceinline__ static constexpr int at(int f, int t, int u) { return f * REGION + (row(t) * PP + u) * 16; }
-    static constexpr int NTW = (RA - 1) * Q;  // first-stage twiddles, staged after the tile
+template <typename C, int NT_> struct LineGeom {
+    static constexpr int NT = NT_;
+    static constexpr LineShape S = tpass_line_shape(NT);
+    static constexpr int RA = S.ra, RB = S.rb, RC = S.rc, PP = S.pp, THREADS = S.threads, MINB = S.ctas;
+    static constexpr int PX = LineUnit<C>::PX;
+    static constexpr int P = PP * PX;            // pixels per tile
+    static constexpr int Q = NT / RA;            // butterflies per line of the first stage
+    static constexpr int RL = RC > 1 ? RC : RB;  // radix of the last forward stage
+    static constexpr int NG = NT / RL;           // its butterflies per line
+    static constexpr bool PAD = PP == 4 && RC == 1;
+    static constexpr int MASK = !PAD && PP < 8 ? 8 / PP - 1 : 0;
+    static constexpr int REGION = (NT + (PAD ? NG : 0)) * PP * 16;  // bytes per field region
+    static constexpr int A = PP * Q;             // first-stage items per field
+    static constexpr int B = PP * (NT / RB);     // middle-stage items (three radices)
+    static constexpr int LAST = PP * NG;         // last-stage items
+    static constexpr int NTW = (RA - 1) * Q;     // first-stage twiddles, staged after the tile
     static constexpr int TILE_BYTES = 3 * REGION;
     static constexpr size_t tile_bytes() { return (size_t)TILE_BYTES + (size_t)NTW * sizeof(C); }
+    static_assert(RL % (MASK + 1) == 0, "rows permute inside a group");
+    // shared-memory row of sample g RL + k, and byte offset of (row, unit) in a field region
+    __device__ __forceinline__ static constexpr int row(int g, int k) { return PAD ? g * (RL + 1) + k : g * RL + (k ^ (g & MASK)); }
+    __device__ __forceinline__ static constexpr int off(int row, int u) { return (row * PP + u) * 16; }
 };
 
-// Issue the cp.async copies of tile `tile` (the fields in lmask) into buffer buf.
-template <typename C, int NT, int RA, int THREADS>
-__device__ __forceinline__ void line_stage_in(const TPassArgs<C> &a, unsigned tile, unsigned lmask, unsigned char *buf)
+// Issue the cp.async copies of a tile (the fields in lmask) into buffer buf.
+template <typename C, typename G>
+__device__ __forceinline__ void line_stage_in(const TPassArgs<C> &a, unsigned base, unsigned lmask, unsigned char *buf)
 {
-    using G = LineGeom<C, NT, RA>;
-    const unsigned base = tile_base(a.g, tile), gs = a.g.gs_j;
+    const unsigned gs = a.g.gs_j;
     const C *src[3] = {a.psrc, a.f[1], a.f[2]};
 #pragma unroll
     for (int f = 0; f < 3; f++) {
         if (!(lmask & (1u << f))) continue;
         const C *gsrc = src[f] + base;
-        for (unsigned e = threadIdx.x; e < NT * G::PP; e += THREADS) {
+        for (unsigned e = threadIdx.x; e < G::NT * G::PP; e += G::THREADS) {
             const int t = (int)(e / G::PP), u = (int)(e % G::PP);
-            cp_async<16>(buf + G::at(f, t, u), gsrc + (size_t)t * gs + u * LineUnit<C>::PX);
+            cp_async<16>(buf + f * G::REGION + G::off(G::row(t / G::RL, t % G::RL), u),
+                         gsrc + (size_t)t * gs + u * G::PX);
         }
     }
 }
@@ -280,18 +369,20 @@ __device__ __forceinline__ void line_stage_in(const TPassArgs<C> &a, unsigned ti
 // Sweep over the staged tile: half steps and EOM per unit, two units per thread at a time
 // (items e and e + THREADS: two independent chains to interleave); transformed fields go
 // back to shared memory as units, the others (loaded, not transformed) to global memory.
-template <typename C, int NT, int RA, int THREADS>
-__device__ __forceinline__ void line_sweep(const TPassArgs<C> &a, unsigned base, unsigned lmask, unsigned tmask,
-                                           unsigned char *buf)
+template <typename C, typename G>
+__device__ __forceinline__ void line_sweep(const TPassArgs<C> &a, unsigned base, unsigned lmask, unsigned tmask, unsigned char *buf)
 {
-    using G = LineGeom<C, NT, RA>;
     using L = LineUnit<C>;
     using U = typename L::U;
+    constexpr unsigned THREADS = G::THREADS;
     const unsigned gs = a.g.gs_j;
-    auto load = [&](unsigned e, U (&v)[3]) {
+    auto at = [&](int f, unsigned e) {
         const int t = (int)(e / G::PP), u = (int)(e % G::PP);
+        return buf + f * G::REGION + G::off(G::row(t / G::RL, t % G::RL), u);
+    };
+    auto load = [&](unsigned e, U (&v)[3]) {
 #pragma unroll
-        for (int f = 0; f < 3; f++) v[f] = (lmask & (1u << f)) ? L::load_raw(buf + G::at(f, t, u)) : L::zero();
+        for (int f = 0; f < 3; f++) v[f] = (lmask & (1u << f)) ? L::load_raw(at(f, e)) : L::zero();
     };
     auto finish = [&](unsigned e, U (&v)[3]) {
         const int t = (int)(e / G::PP), u = (int)(e % G::PP);
@@ -303,12 +394,12 @@ __device__ __forceinline__ void line_sweep(const TPassArgs<C> &a, unsigned base,
 #pragma unroll
         for (int f = 0; f < 3; f++) {
             if (tmask & (1u << f))
-                L::sts(buf + G::at(f, t, u), v[f]);
+                L::sts(at(f, e), v[f]);
             else if (lmask & (1u << f))
-                L::store_raw(a.f[f] + base + (unsigned)t * gs + u * L::PX, v[f]);
+                L::store_raw(a.f[f] + base + (unsigned)t * gs + u * G::PX, v[f]);
         }
     };
-    constexpr unsigned NI = NT * G::PP;
+    constexpr unsigned NI = G::NT * G::PP;
     for (unsigned e = threadIdx.x; e < NI; e += 2 * THREADS) {
         const bool two = e + THREADS < NI;
         U v0[3], v1[3];
@@ -321,140 +412,167 @@ __device__ __forceinline__ void line_sweep(const TPassArgs<C> &a, unsigned base,
     }
 }
 
-// Item w of field f in the forward RA-point stage (stride Q): butterfly, then the
-// twiddles W_NT^{j k}.
-template <typename C, int NT, int RA>
-__device__ __forceinline__ void line_stage_a(const TPassArgs<C> &a, unsigned char *buf, int f, unsigned w)
+// Row of first-stage value m of butterfly j (sample j + Q m).  Q is a multiple of RL: the
+// group is j / RL + (Q / RL) m; with two stages j < Q = RL and the group is m.
+template <typename G> __device__ __forceinline__ int line_row_a(int j, int m)
 {
-    using G = LineGeom<C, NT, RA>;
+    if constexpr (G::RC == 1) return G::row(m, j);
+    return G::row(j / G::RL + G::Q / G::RL * m, j % G::RL);
+}
+
+// Item w of a field in the forward first stage (stride Q): butterfly, then the twiddles
+// W_NT^{j k}.
+template <typename C, typename G>
+__device__ __forceinline__ void line_stage_a(const unsigned char *tws_, unsigned char *buf, unsigned w)
+{
     using L = LineUnit<C>;
-    constexpr int Q = G::Q;
+    constexpr int Q = G::Q, RA = G::RA;
     const int u = (int)(w % G::PP), j = (int)(w / G::PP);
     typename L::U x[RA];
 #pragma unroll
-    for (int m = 0; m < RA; m++) x[m] = L::lds(buf + G::at(f, j + Q * m, u));
+    for (int m = 0; m < RA; m++) x[m] = L::lds(buf + G::off(line_row_a<G>(j, m), u));
     L::template dft<RA, +1>(x);
-    const C *tws = reinterpret_cast<const C *>(buf + G::TILE_BYTES);
+    const C *tws = reinterpret_cast<const C *>(tws_);
 #pragma unroll
     for (int k = 1; k < RA; k++) x[k] = L::template tmul<true>(x[k], tws[(k - 1) * Q + j]);
 #pragma unroll
-    for (int k = 0; k < RA; k++) L::sts(buf + G::at(f, j + Q * k, u), x[k]);
+    for (int k = 0; k < RA; k++) L::sts(buf + G::off(line_row_a<G>(j, k), u), x[k]);
 }
 
-// Item w of field f in the RB-point stage: butterfly, phase table, inverse butterfly.
-template <typename C, int NT, int RA>
-__device__ __forceinline__ void line_stage_b(const TPassArgs<C> &a, unsigned char *buf, int f, unsigned w)
+// Item w of a field in the middle stage of a three-radix plan (stride RC inside blocks of
+// Q samples), forward or inverse.
+template <typename C, typename G, bool FWD>
+__device__ __forceinline__ void line_stage_m(const C *tw1, unsigned char *buf, unsigned w)
 {
-    using G = LineGeom<C, NT, RA>;
     using L = LineUnit<C>;
-    constexpr int RB = G::RB;
-    const int u = (int)(w % G::PP), g = (int)(w / G::PP);
-    unsigned char *sp = buf + G::at(f, RB * g, u);
-    const C *tb = a.tab[f] + RB * g;
+    constexpr int RB = G::RB, RC = G::RC;
+    const int u = (int)(w % G::PP), b = (int)(w / G::PP), blk = b / RC, j = b % RC;
     typename L::U x[RB];
 #pragma unroll
-    for (int m = 0; m < RB; m++) x[m] = L::lds(sp + m * G::PP * 16);
-    L::template dft<RB, +1>(x);
-    if constexpr (sizeof(C) == 8) {
-        // two FP32 table entries per 16-byte load (tb is 16-byte aligned: RB g even)
+    for (int m = 0; m < RB; m++) x[m] = L::lds(buf + G::off(G::row(blk * RB + m, j), u));
+    if constexpr (!FWD) {
 #pragma unroll
-        for (int k = 0; k < RB; k += 2) {
+        for (int m = 1; m < RB; m++) x[m] = L::template tmul<false>(x[m], __ldg(tw1 + (m - 1) * RC + j));
+    }
+    L::template dft<RB, FWD ? +1 : -1>(x);
+    if constexpr (FWD) {
+#pragma unroll
+        for (int k = 1; k < RB; k++) x[k] = L::template tmul<true>(x[k], __ldg(tw1 + (k - 1) * RC + j));
+    }
+#pragma unroll
+    for (int k = 0; k < RB; k++) L::sts(buf + G::off(G::row(blk * RB + k, j), u), x[k]);
+}
+
+// Item w of a field in the last forward stage: butterfly, phase table, inverse butterfly.
+template <typename C, typename G>
+__device__ __forceinline__ void line_stage_b(const C *tab, unsigned char *buf, unsigned w)
+{
+    using L = LineUnit<C>;
+    constexpr int RL = G::RL;
+    const int u = (int)(w % G::PP), g = (int)(w / G::PP);
+    const C *tb = tab + RL * g;
+    typename L::U x[RL];
+#pragma unroll
+    for (int m = 0; m < RL; m++) x[m] = L::lds(buf + G::off(G::row(g, m), u));
+    L::template dft<RL, +1>(x);
+    if constexpr (sizeof(C) == 8) {
+        // two FP32 table entries per 16-byte load (tb is 16-byte aligned: RL g even)
+#pragma unroll
+        for (int k = 0; k < RL; k += 2) {
             const float4 t2 = __ldg(reinterpret_cast<const float4 *>(tb + k));
             x[k] = L::template tmul<false>(x[k], C{t2.x, t2.y});
             x[k + 1] = L::template tmul<false>(x[k + 1], C{t2.z, t2.w});
         }
     } else {
 #pragma unroll
-        for (int k = 0; k < RB; k++) x[k] = L::template tmul<false>(x[k], __ldg(tb + k));
+        for (int k = 0; k < RL; k++) x[k] = L::template tmul<false>(x[k], __ldg(tb + k));
     }
-    L::template dft<RB, -1>(x);
+    L::template dft<RL, -1>(x);
 #pragma unroll
-    for (int k = 0; k < RB; k++) L::sts(sp + k * G::PP * 16, x[k]);
+    for (int k = 0; k < RL; k++) L::sts(buf + G::off(G::row(g, k), u), x[k]);
 }
 
-// Item w of field f in the inverse RA-point stage (twiddles before the butterfly),
-// written to global memory.
-template <typename C, int NT, int RA>
-__device__ __forceinline__ void line_stage_c(const TPassArgs<C> &a, const unsigned char *buf, int f, unsigned w,
-                                             unsigned base, unsigned gs)
+// Item w of a field in the inverse first stage (twiddles before the butterfly), written to
+// global memory.
+template <typename C, typename G>
+__device__ __forceinline__ void line_stage_c(const unsigned char *tws_, const unsigned char *buf, C *dst, unsigned w, unsigned gs)
 {
-    using G = LineGeom<C, NT, RA>;
     using L = LineUnit<C>;
-    constexpr int Q = G::Q;
+    constexpr int Q = G::Q, RA = G::RA;
     const int u = (int)(w % G::PP), j = (int)(w / G::PP);
     typename L::U x[RA];
 #pragma unroll
-    for (int m = 0; m < RA; m++) x[m] = L::lds(buf + G::at(f, j + Q * m, u));
-    const C *tws = reinterpret_cast<const C *>(buf + G::TILE_BYTES);
+    for (int m = 0; m < RA; m++) x[m] = L::lds(buf + G::off(line_row_a<G>(j, m), u));
+    const C *tws = reinterpret_cast<const C *>(tws_);
 #pragma unroll
     for (int m = 1; m < RA; m++) x[m] = L::template tmul<false>(x[m], tws[(m - 1) * Q + j]);
     L::template dft<RA, -1>(x);
-    C *d = a.f[f] + base + (unsigned)j * gs + u * L::PX;
+    C *d = dst + (unsigned)j * gs + u * G::PX;
 #pragma unroll
     for (int k = 0; k < RA; k++) L::store_raw(d + (size_t)(Q * k) * gs, x[k]);
 }
 
-// The three transform stages of every field in tmask as jobs (stage, field) in
-// stage-major order, two jobs per phase (half the CTA each; one job when one field is
-// transformed) and a CTA barrier between phases.  A job's stage of a field always ran
-// in an earlier phase (nf >= 2 jobs apart), and three fields take five phases of whole
-// warps instead of three stages that leave half the warps idle for their second half.
-template <typename C, int NT, int RA, int THREADS, int BAR, int PER>
-__device__ __forceinline__ void line_jobs(const TPassArgs<C> &a, unsigned base, unsigned tmask, unsigned nf,
-                                          unsigned char *buf)
+// The transform stages of every field in tmask as jobs (stage, field) in stage-major
+// order, two jobs per phase (half the CTA each; one job when one field is transformed)
+// and a CTA barrier between phases.  A job's stage of a field always ran in an earlier
+// phase (nf >= 2 jobs apart), and three fields take ceil(3 stages / 2) phases of whole
+// warps instead of one round per stage that leaves half the warps idle for its second half.
+template <typename C, typename G, int BAR, int PER>
+__device__ __forceinline__ void line_jobs(const TPassArgs<C> &a, unsigned base, unsigned tmask, unsigned nf, unsigned char *buf)
 {
-    using G = LineGeom<C, NT, RA>;
-    constexpr unsigned GROUP = THREADS / PER;
-    const unsigned gs = a.g.gs_j, njobs = 3 * nf;
+    constexpr unsigned GROUP = G::THREADS / PER, STAGES = G::RC > 1 ? 5 : 3;
+    static_assert(GROUP % 32 == 0, "a warp runs one job");
+    const unsigned gs = a.g.gs_j, njobs = STAGES * nf;
     const unsigned slot = threadIdx.x / GROUP, w0 = threadIdx.x % GROUP;
+    const unsigned char *tws = buf + G::TILE_BYTES;
     for (unsigned j0 = 0; j0 < njobs; j0 += PER) {
         const unsigned j = j0 + slot;
         if (j < njobs) {
-            // stage j / nf and field j % nf for nf = 1, 2, 3 (j < 9: j / 3 = (11 j) >> 5)
+            // stage j / nf and field j % nf for nf = 1, 2, 3 (j < 15: j / 3 = (11 j) >> 5)
             const unsigned stage = nf == 1 ? j : (nf == 2 ? j >> 1 : (11 * j) >> 5);
             const int f = field_id(tmask, (int)(j - stage * nf));
+            unsigned char *fb = buf + f * G::REGION;
             if (stage == 0) {
-                for (unsigned w = w0; w < G::A; w += GROUP) line_stage_a<C, NT, RA>(a, buf, f, w);
-            } else if (stage == 1) {
-                for (unsigned w = w0; w < G::B; w += GROUP) line_stage_b<C, NT, RA>(a, buf, f, w);
-            } else {
-                for (unsigned w = w0; w < G::A; w += GROUP) line_stage_c<C, NT, RA>(a, buf, f, w, base, gs);
+                for (unsigned w = w0; w < G::A; w += GROUP) line_stage_a<C, G>(tws, fb, w);
+            } else if (stage == STAGES - 1) {
+                for (unsigned w = w0; w < G::A; w += GROUP) line_stage_c<C, G>(tws, fb, a.f[f] + base, w, gs);
+            } else if (G::RC == 1 || stage == 2) {
+                for (unsigned w = w0; w < G::LAST; w += GROUP) line_stage_b<C, G>(a.tab[f], fb, w);
+            } else if constexpr (G::RC > 1) {
+                const C *tw1 = a.tw + G::NTW;
+                if (stage == 1)
+                    for (unsigned w = w0; w < G::B; w += GROUP) line_stage_m<C, G, true>(tw1, fb, w);
+                else
+                    for (unsigned w = w0; w < G::B; w += GROUP) line_stage_m<C, G, false>(tw1, fb, w);
             }
         }
         tile_sync<BAR>();
     }
 }
 
-template <typename C, int NT, int RA, int THREADS, int BAR>
-__device__ __forceinline__ void line_transforms(const TPassArgs<C> &a, unsigned base, unsigned tmask, unsigned char *buf)
-{
-    const unsigned nf = __popc(tmask);
-    if (nf >= 2)
-        line_jobs<C, NT, RA, THREADS, BAR, 2>(a, base, tmask, nf, buf);
-    else
-        line_jobs<C, NT, RA, THREADS, BAR, 1>(a, base, tmask, nf, buf);
-}
-
 // One tile: the fields in the load mask staged with cp.async, the sweep, then per
-// transformed field the RA-point stage, the fused RB-point stage with the phase table,
-// and the inverse RA-point stage written to global memory.  Ends with the CTA
-// synchronised.
-template <typename C, int NT, int RA, int THREADS, int BAR = 0>
+// transformed field the transform stages, the last one written to global memory.  Ends
+// with the CTA synchronised.
+template <typename C, typename G, int BAR = 0>
 __device__ __forceinline__ void tpass_line_tile(const TPassArgs<C> &a, unsigned tile, unsigned char *buf)
 {
-    const unsigned base = tile_base(a.g, tile);
+    const unsigned base = tile * (unsigned)G::P;
     const unsigned tmask = a.tmask, lmask = tpass_load_mask(a);
-    line_stage_in<C, NT, RA, THREADS>(a, tile, lmask, buf);
+    line_stage_in<C, G>(a, base, lmask, buf);
     {  // the first stage's twiddles
-        using G = LineGeom<C, NT, RA>;
         C *tws = reinterpret_cast<C *>(buf + G::TILE_BYTES);
-        for (int e = threadIdx.x; e < G::NTW; e += THREADS) cp_async<sizeof(C)>(tws + e, a.tw + e);
+        for (int e = threadIdx.x; e < G::NTW; e += G::THREADS) cp_async<sizeof(C)>(tws + e, a.tw + e);
     }
     cp_async_wait_all();
     tile_sync<BAR>();
-    line_sweep<C, NT, RA, THREADS>(a, base, lmask, tmask, buf);
+    line_sweep<C, G>(a, base, lmask, tmask, buf);
     tile_sync<BAR>();
-    if (tmask) line_transforms<C, NT, RA, THREADS, BAR>(a, base, tmask, buf);
+    if (!tmask) return;
+    const unsigned nf = __popc(tmask);
+    if (nf >= 2)
+        line_jobs<C, G, BAR, 2>(a, base, tmask, nf, buf);
+    else
+        line_jobs<C, G, BAR, 1>(a, base, tmask, nf, buf);
 }
 
 }  // namespace opo

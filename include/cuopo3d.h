@@ -260,10 +260,12 @@ int opo_set_tuning(OpoSolver *s, const int tuning[9]);
  * kernels: 128 or 256 consumer threads plus one producer warp that streams the tiles
  * into a two-stage shared-memory ring with TMA (t- and y-passes in both precisions,
  * x-pass in FP64); batches run such a setting as its consumer CTA size.  A t-pass radix
- * with OPO_TUNE_LINE added (128 threads) selects the line-specialised t-pass: compiled
- * bodies for the time axes 64, 128 and 256, tiles of 8 FP32 pixels (two per packed
- * instruction) or 4 FP64 pixels; other grids (and the shipped Q2 launch grid) run the
- * generic kernel of the same size with the fallback radix (FP32: the given radix, FP64:
+ * with OPO_TUNE_LINE added (128 threads) selects the line-specialised t-pass also for the
+ * time axes 64, 128 and 256 (nx a multiple of 8 FP32 or 4 FP64 pixels); the time axes 32, 36,
+ * 48, 72, 96, 108, 144, 192, 216, 288, 384, 432, 512, 576, 768, 864 and 1024 run it under every
+ * setting of 128 or 256 threads where a plane holds whole tiles (4 to 16 pixels).  Other
+ * grids (and the shipped Q2 launch grid) run the generic kernel; a line setting's has
+ * its size and the fallback radix (FP32: the given radix, FP64:
  * 4).  x- and y-passes whose axis length has a compiled body (16, 24, 32, 36, 48, 64, 72, 96,
  * 108, 128, 144, 192, 216, 256, 384, 512) run it under every setting of 128 or 256 threads;
  * such a setting's tile and radix then matter to other lengths only.  No counterpart in
