@@ -330,6 +330,11 @@ struct OpoSolver {
     size_t V = 0;
     size_t esz = 0;  // bytes per complex element
     void *field[4] = {};  // Api, Ap, As, Ai
+    // one block: the four fields, the sums, and an area for the first configuration's tables
+    void *mem = nullptr;
+    bool own_mem = true;  // false: a batch's, which outlives the solver
+    char *table_area = nullptr;
+    size_t table_left = 0;
     PassCfg pass[3];
     PlaneCfg plane;
     int *err_dev = nullptr;  // error word of the warp-specialised passes
@@ -448,18 +453,41 @@ template <typename C> C to_c(const cd &v);
 template <> float2 to_c<float2>(const cd &v) { return make_float2((float)v.real(), (float)v.imag()); }
 template <> double2 to_c<double2>(const cd &v) { return make_double2(v.real(), v.imag()); }
 
-template <typename C> int upload(OpoSolver *s, std::vector<void *> &allocs, const std::vector<cd> &h, void **out)
-{
-    std::vector<C> tmp(h.size());
-    for (size_t k = 0; k < h.size(); k++) tmp[k] = to_c<C>(h[k]);
-    void *d = nullptr;
-    OPO_CU(s, cudaMalloc(&d, sizeof(C) * (tmp.size() ? tmp.size() : 1)), "cudaMalloc(table)");
-    allocs.push_back(d);
-    if (!tmp.empty())
-        OPO_CU(s, cudaMemcpy(d, tmp.data(), sizeof(C) * tmp.size(), cudaMemcpyHostToDevice), "cudaMemcpy(table)");
-    *out = d;
-    return OPO_OK;
-}
+// Tables of one configuration, gathered on the host and uploaded together, in stream order:
+// into what is left of the table area of the solver's memory block, else into an
+// allocation of their own (a cudaMalloc / cudaFree pair takes 55 us up to 64 KB and 700 us
+// from 1 MB on, and the free waits for the device; a solver's passes have about 25 tables).
+class TableSet {
+public:
+    // table h, rounded to C, whose device address goes to *out at upload()
+    template <typename C> void add(const std::vector<cd> &h, void **out)
+    {
+        const size_t at = bytes_.size();
+        bytes_.resize(at + (sizeof(C) * (h.empty() ? 1 : h.size()) + 255) / 256 * 256);
+        C *d = reinterpret_cast<C *>(bytes_.data() + at);
+        for (size_t k = 0; k < h.size(); k++) d[k] = to_c<C>(h[k]);
+        slots_.push_back({out, at});
+    }
+    int upload(OpoSolver *s, std::vector<void *> &allocs)
+    {
+        void *mem = nullptr;
+        if (s->table_left >= bytes_.size()) {
+            mem = s->table_area;
+            s->table_area += bytes_.size();
+            s->table_left -= bytes_.size();
+        } else {
+            OPO_CU(s, cudaMalloc(&mem, bytes_.size()), "cudaMalloc(tables)");
+            allocs.push_back(mem);
+        }
+        OPO_CU(s, cudaMemcpyAsync(mem, bytes_.data(), bytes_.size(), cudaMemcpyHostToDevice, s->stream), "copy(tables)");
+        for (auto &sl : slots_) *sl.first = static_cast<char *>(mem) + sl.second;
+        return OPO_OK;
+    }
+
+private:
+    std::vector<unsigned char> bytes_;
+    std::vector<std::pair<void **, size_t>> slots_;
+};
 
 int largest_divisor_leq(int n, int cap)
 {
@@ -786,7 +814,8 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
         cudaError_t e = kind == kX ? opo::configure_axis_line_t<C, true>(n) : opo::configure_axis_line_t<C, false>(n);
         if (e != cudaSuccess) return cuda_fail(s, e, "configure line-specialised axis pass");
     }
-    if ((rc = upload<C>(s, pc.allocs, tw, &pc.tw))) { free_pass(pc); return rc; }
+    TableSet set;
+    set.add<C>(tw, &pc.tw);
     const bool phys = (p.flags & OPO_PHYSICS) != 0;
     const opo::AxisPlan &pl = pc.plan;
     // FP32: every table of this plan carries the transform pair's gain compensation
@@ -815,7 +844,7 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
                 tab[pos] = v * (q2scale / nt);
             }
             fix(tab);
-            if ((rc = upload<TT>(s, pc.allocs, tab, &pc.tab[0][f]))) { free_pass(pc); return rc; }
+            set.add<TT>(tab, &pc.tab[0][f]);
         }
         // GDD compensation exp(i w^2 GDD / 2) (Solver3D.cuh:261-277, 676) times the mirror
         // sqrt(R) e^{i phase} (Cavity3D.cuh:12-28) for resonant signal / idler, / nt
@@ -829,7 +858,7 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
                 tab[pos] = std::polar(1.0, 0.5 * wk * wk * p.gdd) * mirror / (double)nt;
             }
             fix(tab);
-            if ((rc = upload<TT>(s, pc.allocs, tab, &pc.tab[1][f]))) { free_pass(pc); return rc; }
+            set.add<TT>(tab, &pc.tab[1][f]);
         }
         if (p.eom_beta != 0) {
             // EOM exp(i beta sin(2 pi fpm t)) on the t grid (Solver1D.cuh:63-72, t of
@@ -838,7 +867,7 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
             opo_time_freq(nt, p.t_window, tt.data(), nullptr);
             std::vector<cd> e(nt);
             for (int k = 0; k < nt; k++) e[k] = std::polar(1.0, p.eom_beta * std::sin(2 * kPi * p.eom_fpm * tt[k]));
-            if ((rc = upload<C>(s, pc.allocs, e, &pc.eom))) { free_pass(pc); return rc; }
+            set.add<C>(e, &pc.eom);
         }
     } else {
         std::vector<cd> crys[3], free[3];
@@ -847,13 +876,12 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
             fix(crys[f]);
             fix(free[f]);
         }
-        for (int f = 0; f < 3; f++)
-            if ((rc = upload<TT>(s, pc.allocs, crys[f], &pc.tab[0][f])) ||
-                (rc = upload<TT>(s, pc.allocs, free[f], &pc.tab[1][f]))) {
-                free_pass(pc);
-                return rc;
-            }
+        for (int f = 0; f < 3; f++) {
+            set.add<TT>(crys[f], &pc.tab[0][f]);
+            set.add<TT>(free[f], &pc.tab[1][f]);
+        }
     }
+    if ((rc = set.upload(s, pc.allocs))) { free_pass(pc); return rc; }
     pc.grid = g.ntiles;
     if (ws) {
         // persistent: every resident CTA, at most one per tile
@@ -916,10 +944,9 @@ template <typename C> int configure_plane(OpoSolver *s, int K, int threads, int 
     if (opo::plane_max_clusters<C>(threads, K, pc.smem) < 1)
         return fail(s, OPO_ERR_INVALID, "no cluster of the plane pass can be resident");
     int rc;
-    if ((rc = upload<C>(s, pc.allocs, twx, &pc.twx)) || (rc = upload<C>(s, pc.allocs, twy, &pc.twy))) {
-        free_plane(pc);
-        return rc;
-    }
+    TableSet set;
+    set.add<C>(twx, &pc.twx);
+    set.add<C>(twy, &pc.twy);
     std::vector<cd> crys[3], free[3];
     // FP32: the same gain compensation as the separate x / y passes' tables
     std::vector<double> comp;
@@ -929,24 +956,24 @@ template <typename C> int configure_plane(OpoSolver *s, int K, int threads, int 
         opo::scale_table(crys[f], comp);
         opo::scale_table(free[f], comp);
     }
-    for (int f = 0; f < 3; f++)
-        if ((rc = upload<TT>(s, pc.allocs, crys[f], &pc.tabx[0][f])) ||
-            (rc = upload<TT>(s, pc.allocs, free[f], &pc.tabx[1][f]))) {
-            free_plane(pc);
-            return rc;
-        }
+    for (int f = 0; f < 3; f++) {
+        set.add<TT>(crys[f], &pc.tabx[0][f]);
+        set.add<TT>(free[f], &pc.tabx[1][f]);
+    }
     diffraction_tables(p, false, pc.py, crys, free);
     if (!fp64) comp = opo::fp32_pair_compensation(pc.py, twy);
     for (int f = 0; f < 3 && !comp.empty(); f++) {
         opo::scale_table(crys[f], comp);
         opo::scale_table(free[f], comp);
     }
-    for (int f = 0; f < 3; f++)
-        if ((rc = upload<TT>(s, pc.allocs, crys[f], &pc.taby[0][f])) ||
-            (rc = upload<TT>(s, pc.allocs, free[f], &pc.taby[1][f]))) {
-            free_plane(pc);
-            return rc;
-        }
+    for (int f = 0; f < 3; f++) {
+        set.add<TT>(crys[f], &pc.taby[0][f]);
+        set.add<TT>(free[f], &pc.taby[1][f]);
+    }
+    if ((rc = set.upload(s, pc.allocs))) {
+        free_plane(pc);
+        return rc;
+    }
     drop_graphs(s);
     free_plane(s->plane);
     s->plane = pc;
@@ -1658,7 +1685,7 @@ int opo_noise(uint64_t seed, double sigma, size_t n, double *out)
 }
 
 static int create_impl(const OpoParams *p, const double *w, const opo::PassVariant *vv, const size_t *tt,
-                       cudaStream_t ext_stream, OpoSolver **out)
+                       cudaStream_t ext_stream, void *block, size_t block_bytes, OpoSolver **out)
 {
     if (!out) return OPO_ERR_INVALID;
     *out = nullptr;
@@ -1685,18 +1712,33 @@ static int create_impl(const OpoParams *p, const double *w, const opo::PassVaria
             rc = cuda_fail(s, e, "stream");
             break;
         }
-        for (int k = 0; k < 4 && !rc; k++) {
-            if ((e = cudaMalloc(&s->field[k], s->esz * s->V)) != cudaSuccess) rc = cuda_fail(s, e, "cudaMalloc(field)");
-            else if ((e = cudaMemset(s->field[k], 0, s->esz * s->V)) != cudaSuccess) rc = cuda_fail(s, e, "memset");
-        }
-        if (rc) break;
-        // The attribute is per kernel function and shared by every solver of the process:
-        // always allow the full 227 KB so no solver lowers it under another.
-        if ((e = cudaMalloc((void **)&s->err_dev, sizeof(int))) != cudaSuccess ||
-            (e = cudaMemset(s->err_dev, 0, sizeof(int))) != cudaSuccess) {
-            rc = cuda_fail(s, e, "cudaMalloc(error word)");
+        const size_t fbytes = (s->esz * s->V + 255) / 256 * 256;
+        // partial sums, the three sums, the error word of the warp-specialised passes
+        s->sum_blocks = 148 * 4;
+        const size_t nsum = 3 * ((size_t)s->sum_blocks + 1), sbytes = (sizeof(double) * nsum + sizeof(int) + 255) / 256 * 256;
+        constexpr size_t kTableArea = 256 * 1024;
+        size_t bytes = 4 * fbytes + sbytes + kTableArea;
+        if (block && block_bytes >= 4 * fbytes + sbytes) {
+            s->mem = block;
+            s->own_mem = false;
+            bytes = block_bytes;
+        } else if ((e = cudaMalloc(&s->mem, bytes)) != cudaSuccess) {
+            rc = cuda_fail(s, e, "cudaMalloc(fields)");
             break;
         }
+        char *m = static_cast<char *>(s->mem);
+        for (int k = 0; k < 4; k++) s->field[k] = m + k * fbytes;
+        s->partials = reinterpret_cast<double *>(m + 4 * fbytes);
+        s->sums_dev = s->partials + 3 * s->sum_blocks;
+        s->err_dev = reinterpret_cast<int *>(s->partials + nsum);
+        s->table_area = m + 4 * fbytes + sbytes;
+        s->table_left = bytes - 4 * fbytes - sbytes;
+        if ((e = cudaMemsetAsync(s->mem, 0, 4 * fbytes + sbytes, s->stream)) != cudaSuccess) {
+            rc = cuda_fail(s, e, "memset");
+            break;
+        }
+        // The attribute is per kernel function and shared by every solver of the process:
+        // always allow the full 227 KB so no solver lowers it under another.
         if ((e = opo::configure_kernels(227 * 1024)) != cudaSuccess ||
             (e = opo::configure_plane_kernels(227 * 1024)) != cudaSuccess ||
             (e = opo::configure_ws_kernels(227 * 1024)) != cudaSuccess ||
@@ -1721,12 +1763,6 @@ static int create_impl(const OpoParams *p, const double *w, const opo::PassVaria
             if (rc) break;
         }
         s->gdd_or_mirror = s->p.gdd != 0 || (s->p.resonant & 6u);
-        s->sum_blocks = 148 * 4;
-        if ((e = cudaMalloc((void **)&s->partials, sizeof(double) * 3 * (s->sum_blocks + 1))) != cudaSuccess) {
-            rc = cuda_fail(s, e, "cudaMalloc(partials)");
-            break;
-        }
-        s->sums_dev = s->partials + 3 * s->sum_blocks;
     } while (0);
     if (rc) {
         g_static_err = "opo_create failed";
@@ -1740,7 +1776,7 @@ static int create_impl(const OpoParams *p, const double *w, const opo::PassVaria
 
 int opo_create(const OpoParams *p, const double *w, OpoSolver **out)
 {
-    return create_impl(p, w, nullptr, nullptr, nullptr, out);
+    return create_impl(p, w, nullptr, nullptr, nullptr, nullptr, 0, out);
 }
 
 void opo_destroy(OpoSolver *s)
@@ -1765,11 +1801,8 @@ void opo_destroy(OpoSolver *s)
         if (s->st.in[k]) cudaFree(s->st.in[k]);
         if (s->st.out[k]) cudaFree(s->st.out[k]);
     }
-    for (auto *f : s->field)
-        if (f) cudaFree(f);
-    if (s->partials) cudaFree(s->partials);
+    if (s->mem && s->own_mem) cudaFree(s->mem);
     if (s->staging) cudaFree(s->staging);
-    if (s->err_dev) cudaFree(s->err_dev);
     for (auto &pc : s->pass) free_pass(pc);
     free_plane(s->plane);
     if (s->stream && s->own_stream) cudaStreamDestroy(s->stream);
@@ -2080,9 +2113,9 @@ const char *opo_last_error(const OpoSolver *s) { return s ? s->err.c_str() : g_s
 namespace opo {
 
 int solver_create_configured(const OpoParams *p, const double *w, const PassVariant v[3], const size_t te[3],
-                             cudaStream_t stream, OpoSolver **out)
+                             cudaStream_t stream, void *block, size_t block_bytes, OpoSolver **out)
 {
-    return create_impl(p, w, v, te, stream, out);
+    return create_impl(p, w, v, te, stream, block, block_bytes, out);
 }
 
 PassVariant solver_pass_variant(const OpoSolver *s, int kind) { return s->pass[kind].v; }

@@ -17,9 +17,11 @@ inline size_t batch_instance_bytes(int precision, size_t voxels)
 }
 
 // Create a solver with the given kernel variant and tile size per pass (t, x, y);
-// `stream` (may be null) replaces the solver's own stream, e.g. a batch's stream.
+// `stream` (may be null) replaces the solver's own stream, e.g. a batch's stream, and
+// `block` (may be null) of block_bytes its device memory for fields, sums and tables; the
+// caller keeps both until the solver is destroyed.
 int solver_create_configured(const OpoParams *p, const double *w, const PassVariant v[3], const size_t te[3],
-                             cudaStream_t stream, OpoSolver **out);
+                             cudaStream_t stream, void *block, size_t block_bytes, OpoSolver **out);
 void solver_pass_info(const OpoSolver *s, int kind, int *ntiles, size_t *smem);
 PassVariant solver_pass_variant(const OpoSolver *s, int kind);
 // A line-specialised t-pass setting runs its line body on s's grid, or its generic
