@@ -7,6 +7,7 @@
 #include "fft_gain.h"
 #include "opo_internal.h"
 #include "solver_internal.h"
+#include "wave_pass.h"
 
 #include <cudaTypedefs.h>
 
@@ -292,6 +293,9 @@ struct PassCfg {
     int line_nt = 0;  // t-pass: the line-specialised kernel's time axis (0: generic kernel)
     int line_n = 0;   // x / y: the line-specialised body's axis length (0: generic kernel)
     unsigned line_extent = 0;
+    int wave_K = 0;   // t: the plane-wave kernel's cluster size (wave_pass.cu; 0: pass by pass)
+    int wave_nsample = 0;
+    void *ph_steps = nullptr;  // its exp(i dk z) per t-pass (corrected physics)
     void *tw = nullptr;
     void *tab[2][3] = {};
     void *eom = nullptr;  // t-pass: EOM phase per time sample (natural order), or null
@@ -333,6 +337,7 @@ struct OpoSolver {
     // one block: the four fields, the sums, and an area for the first configuration's tables
     void *mem = nullptr;
     bool own_mem = true;  // false: a batch's, which outlives the solver
+    bool batched = false;  // a batch's instance: run pass by pass by the batch's kernels
     char *table_area = nullptr;
     size_t table_left = 0;
     PassCfg pass[3];
@@ -591,7 +596,8 @@ void default_variant(const OpoParams &p, int kind, opo::PassVariant &v, size_t &
 {
     const bool fp64 = p.precision == OPO_FP64;
     const opo::PassVariant line{128, opo::kLineForm | (fp64 ? 4 : 16)};
-    if (kind == kT && (fp64 ? tpass_line_body<double2>(p, line) : tpass_line_body<float2>(p, line))) {
+    const bool wave = p.nx == 1 && p.ny == 1 && !(p.flags & (OPO_DIFFRACTION | OPO_ASIS_Q2));
+    if (kind == kT && (wave || (fp64 ? tpass_line_body<double2>(p, line) : tpass_line_body<float2>(p, line)))) {
         v = line;
         te = fp64 ? 1024 : 2048;
         return;
@@ -660,6 +666,61 @@ template <typename C> bool use_tpass_line(const OpoParams &p, PassCfg &pc, std::
     pc.line_nt = p.nt;
     pc.smem = opo::tpass_line_smem<C>(p.nt);
     return true;
+}
+
+// Whether a solver's crystal runs as one launch of the plane-wave kernel under t-setting v: a
+// single time line and no diffraction.  (The other settings, and a batch, keep the t-pass.)
+bool wave_setting(const OpoSolver *s, opo::PassVariant v)
+{
+    const OpoParams &p = s->p;
+    return opo::is_line(v) && !s->batched && p.nx == 1 && p.ny == 1 && !(p.flags & (OPO_DIFFRACTION | OPO_ASIS_Q2));
+}
+
+// Plan, cluster size and geometry of the plane-wave kernel; false when none fits (the t-pass
+// stays).  K CTAs divide the line's arithmetic and pay two cluster barriers a step: the
+// largest K that the length and the device take from 2048 samples on, fewer for short lines.
+template <typename C> bool use_wave(const OpoSolver *s, PassCfg &pc, std::vector<cd> &tw)
+{
+    const int n = s->p.nt;
+    for (int K : {16, 8, 4, 1}) {
+        if ((K == 16 && n < 2048) || (K == 8 && n < 512) || n % (K * K) || n / K < 4) continue;
+        std::vector<int> rad;
+        if (K == 16) rad = {4, 4};
+        else if (K > 1) rad = {K};
+        const int nsample = (int)rad.size(), M = n / K;
+        int m = M, a = 0;
+        while (m % 2 == 0) { m /= 2; a++; }
+        while (m % 3 == 0) { m /= 3; rad.push_back(3); }
+        if (m != 1 || !split_pow2(a, 8, rad)) continue;
+        opo::AxisPlan plan;
+        std::vector<cd> t;
+        if (!plan_of_radices(n, rad, plan, t)) continue;
+        opo::TileGeom g{};
+        g.nlines = 1;
+        g.ntiles = 1;
+        g.lsl = 1;
+        g.lsj = 1;
+        g.gs_j = g.gs_l = 1;
+        g.nl = make_fastdiv(1);
+        const int R = plan.radix[plan.ns - 1];
+        unsigned rows = (unsigned)M;
+        if ((R & (R - 1)) == 0) {
+            g.psh = 0;
+            while ((1 << g.psh) < R) g.psh++;
+            rows += (unsigned)M >> g.psh;
+        }
+        g.region = (rows + 1u) & ~1u;
+        const size_t smem = 3 * sizeof(C) * ((size_t)g.region + (K > 1 ? M : 0));
+        if (!opo::wave_fits<C>(K, smem)) continue;
+        pc.plan = plan;
+        tw = t;
+        pc.geo = g;
+        pc.smem = smem;
+        pc.wave_K = K;
+        pc.wave_nsample = nsample;
+        return true;
+    }
+    return false;
 }
 
 // Build the plan, geometry and tables of one pass kind for variant v and tile size te.
@@ -748,6 +809,11 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
         g.region = (g.region + per128 - 1) / per128 * per128;
     }
     pc.smem = 3 * (size_t)g.region * sizeof(C);
+    if (kind == kT && wave_setting(s, v)) {
+        cudaError_t e = opo::configure_wave_kernels<C>();
+        if (e != cudaSuccess) return cuda_fail(s, e, "configure plane-wave kernel");
+        use_wave<C>(s, pc, tw);
+    }
     if (pc.smem > 227 * 1024 && !(line && form)) return fail(s, OPO_ERR_INVALID, "tile does not fit in shared memory");
     if (ws) {
         opo::WsArgs &w = pc.wsa;
@@ -859,6 +925,20 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
             }
             fix(tab);
             set.add<TT>(tab, &pc.tab[1][f]);
+        }
+        if (pc.wave_K && phys && p.dk != 0) {
+            std::vector<cd> ph((size_t)(p.n_steps + 1) * 6);
+            for (int tp = 0; tp <= p.n_steps; tp++) {
+                double zh[2];
+                int nrk;
+                opo::solver_tpass_z(p, tp, zh, &nrk);
+                const double h = 0.5 * p.dz;
+                for (int k = 0; k < 2; k++) {
+                    const double zs[3] = {zh[k], zh[k] + 0.5 * h, zh[k] + h};
+                    for (int j = 0; j < 3; j++) ph[(size_t)tp * 6 + k * 3 + j] = std::polar(1.0, p.dk * zs[j]);
+                }
+            }
+            set.add<C>(ph, &pc.ph_steps);
         }
         if (p.eom_beta != 0) {
             // EOM exp(i beta sin(2 pi fpm t)) on the t grid (Solver1D.cuh:63-72, t of
@@ -1198,6 +1278,36 @@ template <typename C> int enqueue_crystal(OpoSolver *s, bool reset_pump)
     return OPO_OK;
 }
 
+// The crystal and its closing pass in one launch (wave_pass.cu); closing: a round trip's.
+template <typename C> int enqueue_wave(OpoSolver *s, bool reset_pump, bool closing)
+{
+    const OpoParams &p = s->p;
+    const PassCfg &pc = s->pass[kT];
+    opo::WaveArgs<C> w{};
+    const double z0[2] = {0, 0};
+    w.rk = opo::make_tpass_args<C>(s, reset_pump, 1, z0, 0, 7u);
+    w.K = (unsigned)pc.wave_K;
+    w.M = (unsigned)p.nt / w.K;
+    w.bw = w.M / w.K;
+    w.nsample = pc.wave_nsample;
+    w.xregion = w.M;
+    w.plan = pc.plan;
+    w.g = pc.geo;
+    w.tw = static_cast<const C *>(pc.tw);
+    for (int k = 0; k < 2; k++)
+        for (int f = 0; f < 3; f++) w.tab[k][f] = tabs<C>(s, kT, k)[f];
+    w.eom = static_cast<const C *>(pc.eom);
+    w.ph_steps = static_cast<const C *>(pc.ph_steps);
+    w.n_steps = p.n_steps;
+    w.mask = (p.flags & OPO_DISPERSION) ? 7u : 0u;
+    w.closing = closing ? 1 : 0;
+    w.close_mask = s->gdd_or_mirror ? 6u : 0u;
+    PassTimer timer(s, 0);
+    OPO_CU(s, opo::launch_wave<C>(w, pc.smem, s->stream), "plane-wave launch");
+    s->launches++;
+    return OPO_OK;
+}
+
 double last_half_z(const OpoParams &p)
 {
     const int k = p.n_steps - 1;
@@ -1206,6 +1316,7 @@ double last_half_z(const OpoParams &p)
 
 template <typename C> int enqueue_single_pass(OpoSolver *s)
 {
+    if (s->pass[kT].wave_K) return enqueue_wave<C>(s, false, false);
     int rc;
     if ((rc = enqueue_crystal<C>(s, false))) return rc;
     const double z = last_half_z(s->p);
@@ -1218,6 +1329,7 @@ template <typename C> int enqueue_single_pass(OpoSolver *s)
 // space and t-axis operators commute, so GDD + mirrors may precede the return.
 template <typename C> int enqueue_round_trip(OpoSolver *s, bool last)
 {
+    if (s->pass[kT].wave_K) return enqueue_wave<C>(s, true, true);
     const OpoParams &p = s->p;
     int rc;
     if ((rc = enqueue_crystal<C>(s, true))) return rc;
@@ -1397,8 +1509,11 @@ template <typename C> int autotune(OpoSolver *s)
         best.te[kind] = s->pass[kind].te;
         if (kind != kT && !(s->p.flags & OPO_DIFFRACTION)) continue;
         {
-            // a body that runs whatever the classic setting: nothing to time
-            bool line = false;
+            // a body that runs whatever the classic setting, or the plane-wave kernel: nothing
+            // to time
+            const opo::PassVariant lv{128, (fp64 ? 4 : 16) | opo::kLineForm};
+            bool line = kind == kT && wave_setting(s, lv) && configure_pass<C>(s, kind, lv, tes[1]) == OPO_OK &&
+                        s->pass[kind].wave_K;
             for (int r1 : {8, 4})
                 if (!line && configure_pass<C>(s, kind, opo::PassVariant{128, r1}, tes[1]) == OPO_OK)
                     line = (s->pass[kind].line_n || s->pass[kind].line_nt) && s->pass[kind].v.r1 == r1;
@@ -1721,6 +1836,7 @@ static int create_impl(const OpoParams *p, const double *w, const opo::PassVaria
         if (block && block_bytes >= 4 * fbytes + sbytes) {
             s->mem = block;
             s->own_mem = false;
+            s->batched = true;
             bytes = block_bytes;
         } else if ((e = cudaMalloc(&s->mem, bytes)) != cudaSuccess) {
             rc = cuda_fail(s, e, "cudaMalloc(fields)");
