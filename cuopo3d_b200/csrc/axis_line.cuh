@@ -34,6 +34,7 @@
 
 #include "fft_radix.cuh"
 #include "opo_internal.h"
+#include "tma_copy.cuh"
 
 namespace opo {
 
@@ -123,10 +124,19 @@ template <typename C, bool X_, int N_> struct AxisLine {
     static constexpr int RL = RC > 1 ? RC : RB;   // radix of the last forward stage
     static constexpr int NG = N / RL;             // its butterflies per line
     static constexpr int LS = X ? axis_line_stride(N, RA, RB, RC, F64 ? 8 : 16) : 0;
-    static constexpr int BYTES = (X ? L * LS : N * L) * (int)sizeof(C);
+    // TMA-fed tiles (axis_line_load): the raw stride of an x line, for which the first stage's
+    // reads of consecutive elements fill whole wavefronts across lines
+    static constexpr int NB = F64 ? 8 : 16;
+    static constexpr int LSR = N + (Q % NB + NB - N % NB) % NB;
+    static constexpr int BYTES = ((X ? L * (LS > LSR ? LS : LSR) : N * L) * (int)sizeof(C) + 127) / 128 * 128;
     // one first-stage item per thread up to 256 threads, then two
     static constexpr int ITEMS = Q * L;
     static constexpr int THREADS = ((ITEMS <= 256 ? ITEMS : (ITEMS + 1) / 2) + 31) / 32 * 32;
+    // TMA-fed: one item per thread, and from 128 points on -- loads through registers hold their
+    // bytes in flight in L1, which beside the t-pass's shared memory (three solvers in turn, the
+    // SMs' split at its largest) is 28 KB: 128 x 128 x 256 FP32 15.0 -> 14.0 ms a round trip, FP64
+    // 30.3 -> 27.7; alone, and below 128 points, the two are within 1-5 %, registers ahead
+    static constexpr bool TMA = ITEMS <= THREADS && N >= 128;
     // Registers: FP32 80 (at 64 the radix-16 y-pass of ragged grids spills: 47 us against 39),
     // FP64 128 with a radix above 8, else 96.
     static constexpr int REGS = F64 ? (RA > 8 || RB > 8 ? 128 : 96) : X && RA == 16 && RB == 8 ? 64 : 80;
@@ -156,10 +166,21 @@ template <typename C, bool X> inline size_t axis_line_smem(int n)
     }
 }
 
+// Whether the body for n points can be TMA-fed, and its columns per y box.
+template <typename C, bool X> inline bool axis_line_tma(int n)
+{
+    switch (n) {
+#define OPO_CASE(N) case N: return AxisLine<C, X, N>::TMA;
+        OPO_AXIS_LINES(OPO_CASE)
+#undef OPO_CASE
+    default: return false;
+    }
+}
+
 // One tile: lines [0, lim) of the L starting at fp (lim < L: the last tile of a row or
 // field), row stride gs (elements; y: between positions, GS != 0 fixes it at compile time).
 // Offsets within a tile are 32-bit byte counts.  A caller that reuses sm synchronises first.
-template <typename C, typename G, int THREADS, unsigned GS>
+template <typename C, typename G, int THREADS, unsigned GS, bool LOADED = false>
 __device__ __forceinline__ void axis_line_tile(C *fp, unsigned lim, unsigned gs, const C *__restrict__ tab,
                                                const C *__restrict__ tw, C *sm)
 {
@@ -168,6 +189,23 @@ __device__ __forceinline__ void axis_line_tile(C *fp, unsigned lim, unsigned gs,
     constexpr bool FULL = !G::X && GS % L == 0 && GS > 0;  // square grid of whole tiles
     const unsigned gsj = (G::X ? 1u : (GS ? GS : gs)) * (unsigned)sizeof(C), gsl = (G::X ? G::N : 1u) * (unsigned)sizeof(C);
     char *const gp = reinterpret_cast<char *>(fp);
+    if constexpr (LOADED) {
+        // first stage from the raw tile (x: lines LSR apart; y: in place)
+        static_assert(G::ITEMS <= THREADS, "one item per thread");
+        int l, b;
+        G::item(min((int)threadIdx.x, G::ITEMS - 1), Q, l, b);
+        C x[RA];
+#pragma unroll
+        for (int m = 0; m < RA; m++) x[m] = sm[G::X ? l * G::LSR + b + m * Q : (b + m * Q) * L + l];
+        __syncthreads();  // x: the padded tile overlaps the raw one
+        if (threadIdx.x < G::ITEMS) {
+            dft<RA, -1>(x);
+#pragma unroll
+            for (int k = 1; k < RA; k++) x[k] = cmul(x[k], __ldg(tw + (k - 1) * Q + b));
+#pragma unroll
+            for (int k = 0; k < RA; k++) sm[G::at(l, b + k * Q)] = x[k];
+        }
+    } else
 #pragma unroll 1
     for (int w = threadIdx.x; w < G::ITEMS; w += THREADS) {
         int l, b;
@@ -252,6 +290,32 @@ __device__ __forceinline__ void axis_line_tile(C *fp, unsigned lim, unsigned gs,
 #pragma unroll
         for (int k = 0; k < RA; k++) *reinterpret_cast<C *>(gp + (o + k * Q * gsj)) = x[k];
     }
+}
+
+// Brings the raw tile into sm with the TMA: x one bulk copy per line, y one tensor box (L
+// columns of N rows of the plane; columns past the grid read as zero).  Every thread returns
+// when the tile has landed; false when the bounded wait expired.
+template <typename C, typename G>
+__device__ __forceinline__ bool axis_line_load(const C *fp, unsigned lim, const CUtensorMap *map, int c0, int plane, C *sm,
+                                               unsigned long long *bar)
+{
+    if (threadIdx.x == 0) {
+        mbar_init(bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    const unsigned lines = min(lim, (unsigned)G::L);
+    if (threadIdx.x < 32) {
+        if (threadIdx.x == 0) mbar_arrive_expect_tx(bar, (G::X ? lines : (unsigned)G::L) * G::N * (unsigned)sizeof(C));
+        __syncwarp();
+        if constexpr (G::X) {
+            if (threadIdx.x < lines)
+                tma_bulk(sm + threadIdx.x * G::LSR, fp + threadIdx.x * G::N, G::N * (unsigned)sizeof(C), bar);
+        } else {
+            if (threadIdx.x == 0) tma_tensor_3d(sm, map, c0, 0, plane, bar);
+        }
+    }
+    __syncthreads();  // the barrier is initialised
+    return mbar_wait(bar, 0);
 }
 
 // First element and line count of tile `tile` of a line-specialised pass.

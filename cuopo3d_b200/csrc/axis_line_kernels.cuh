@@ -8,11 +8,18 @@
 
 namespace opo {
 
+// Tensor maps of the fields (y: boxes of L columns, N rows) and the error word of the passes'
+// bounded waits.
+struct AxisLineTma {
+    CUtensorMap map[3];
+};
+
 // CTA u of a launch: tile u mod ntiles of the (u / ntiles)-th field of the mask.
-template <typename C, typename G, unsigned GS>
-__global__ void __launch_bounds__(G::THREADS, G::MINB) axis_line_kernel(AxisArgs<C> a)
+template <typename C, typename G, unsigned GS, bool TMA>
+__device__ __forceinline__ void axis_line_cta(const AxisArgs<C> &a, const CUtensorMap *maps, int *err)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    C *sm = reinterpret_cast<C *>(smem_raw);
     unsigned fi = 0, tile = blockIdx.x;
     while (tile >= (unsigned)a.g.ntiles) {
         tile -= (unsigned)a.g.ntiles;
@@ -20,22 +27,51 @@ __global__ void __launch_bounds__(G::THREADS, G::MINB) axis_line_kernel(AxisArgs
     }
     unsigned m = a.tmask;
     while (fi--) m &= m - 1;  // the fi-th field of the mask is the lowest left
-    C *fp = (m & 1u) ? a.f[0] : (m & 2u) ? a.f[1] : a.f[2];
-    const C *tab = (m & 1u) ? a.tab[0] : (m & 2u) ? a.tab[1] : a.tab[2];
+    const int f = (m & 1u) ? 0 : (m & 2u) ? 1 : 2;
+    C *fp = f == 0 ? a.f[0] : f == 1 ? a.f[1] : a.f[2];
+    const C *tab = f == 0 ? a.tab[0] : f == 1 ? a.tab[1] : a.tab[2];
     unsigned lim;
     fp += axis_line_base(a.g, tile, a.line_extent, lim);
-    axis_line_tile<C, G, G::THREADS, GS>(fp, lim, a.g.gs_j, tab, a.tw, reinterpret_cast<C *>(smem_raw));
+    if constexpr (TMA) {
+        const unsigned hi = fdiv(a.g.tdiv, tile), lo = tile - hi * a.g.tdiv.d;
+        unsigned long long *bar = reinterpret_cast<unsigned long long *>(smem_raw + G::BYTES);
+        if (!axis_line_load<C, G>(fp, lim, maps + f, (int)(lo * G::L * (sizeof(C) / 8)), (int)hi, sm, bar)) {
+            if (err) atomicExch(err, 101);
+            mbar_wait(bar, 0);  // the copy must not land in a later CTA's memory
+        }
+    }
+    axis_line_tile<C, G, G::THREADS, GS, TMA>(fp, lim, a.g.gs_j, tab, a.tw, sm);
 }
 
-template <typename C, bool X> const void *axis_line_func(int n, bool square, int *threads)
+template <typename C, typename G, unsigned GS>
+__global__ void __launch_bounds__(G::THREADS, G::MINB) axis_line_kernel(AxisArgs<C> a)
+{
+    axis_line_cta<C, G, GS, false>(a, nullptr, nullptr);
+}
+template <typename C, typename G, unsigned GS>
+__global__ void __launch_bounds__(G::THREADS, G::MINB)
+    axis_line_tma_kernel(AxisArgs<C> a, const __grid_constant__ AxisLineTma t, int *err)
+{
+    axis_line_cta<C, G, GS, G::TMA>(a, t.map, err);
+}
+
+// Kernel of an axis of n points: square: the grid is, tma: TMA-fed (axis_line_tma).
+template <typename C, bool X> const void *axis_line_func(int n, bool square, bool tma, int *threads)
 {
     switch (n) {
 #define OPO_CASE(N)                                                                                 \
     case N: {                                                                                       \
         using G = AxisLine<C, X, N>;                                                                \
         *threads = G::THREADS;                                                                      \
-        if (!X && square) return reinterpret_cast<const void *>(axis_line_kernel<C, G, X ? 0u : (unsigned)N>); \
-        return reinterpret_cast<const void *>(axis_line_kernel<C, G, 0u>);                          \
+        constexpr unsigned SQ = X ? 0u : (unsigned)N;                                               \
+        if constexpr (G::TMA) {                                                                     \
+            if (tma && square) return reinterpret_cast<const void *>(axis_line_tma_kernel<C, G, SQ>); \
+            if (tma) return reinterpret_cast<const void *>(axis_line_tma_kernel<C, G, 0u>);         \
+            return X ? nullptr : reinterpret_cast<const void *>(axis_line_kernel<C, G, 0u>);        \
+        } else {                                                                                    \
+            if (square) return reinterpret_cast<const void *>(axis_line_kernel<C, G, SQ>);          \
+            return reinterpret_cast<const void *>(axis_line_kernel<C, G, 0u>);                      \
+        }                                                                                           \
     }
         OPO_AXIS_LINES(OPO_CASE)
 #undef OPO_CASE
@@ -44,31 +80,35 @@ template <typename C, bool X> const void *axis_line_func(int n, bool square, int
 }
 
 template <typename C, bool X>
-cudaError_t launch_axis_line_t(const AxisArgs<C> &a, bool square, size_t smem, cudaStream_t st)
+cudaError_t launch_axis_line_t(const AxisArgs<C> &a, bool square, const CUtensorMap *maps, int *err, size_t smem, cudaStream_t st)
 {
     int threads = 0;
-    const void *fn = axis_line_func<C, X>(a.plan.n, square, &threads);
+    const void *fn = axis_line_func<C, X>(a.plan.n, square, maps != nullptr, &threads);
     if (!fn) return cudaErrorInvalidValue;
-    void *args[] = {const_cast<AxisArgs<C> *>(&a)};
-    return cudaLaunchKernel(fn, dim3((unsigned)a.g.ntiles * (unsigned)__builtin_popcount(a.tmask)), dim3(threads), args,
-                            smem, st);
+    const dim3 grid((unsigned)a.g.ntiles * (unsigned)__builtin_popcount(a.tmask));
+    if (!maps) {
+        void *args[] = {const_cast<AxisArgs<C> *>(&a)};
+        return cudaLaunchKernel(fn, grid, dim3(threads), args, smem, st);
+    }
+    void *args[] = {const_cast<AxisArgs<C> *>(&a), const_cast<CUtensorMap *>(maps), &err};
+    return cudaLaunchKernel(fn, grid, dim3(threads), args, smem, st);
 }
 
-// Shared memory above the default 48 KB needs the attribute; set once per function.
+// Shared memory above the default 48 KB needs the attribute.
 template <typename C, bool X> cudaError_t configure_axis_line_t(int n)
 {
-    for (int square = 0; square < (X ? 1 : 2); square++) {
+    for (int k = 0; k < 4; k++) {
         int threads = 0;
-        const void *fn = axis_line_func<C, X>(n, square != 0, &threads);
-        if (!fn) return cudaErrorInvalidValue;
-        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        const void *fn = axis_line_func<C, X>(n, k & 1, k & 2, &threads);
+        cudaError_t e = fn ? cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) : cudaSuccess;
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
 
 #define OPO_AXIS_LINE_INSTANCE(C, X)                                                                \
-    template cudaError_t launch_axis_line_t<C, X>(const AxisArgs<C> &, bool, size_t, cudaStream_t);  \
+    template cudaError_t launch_axis_line_t<C, X>(const AxisArgs<C> &, bool, const CUtensorMap *, int *, size_t, \
+                                                  cudaStream_t);                                    \
     template cudaError_t configure_axis_line_t<C, X>(int);
 
 }  // namespace opo

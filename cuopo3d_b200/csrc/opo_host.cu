@@ -293,6 +293,7 @@ struct PassCfg {
     int line_nt = 0;  // t-pass: the line-specialised kernel's time axis (0: generic kernel)
     int line_n = 0;   // x / y: the line-specialised body's axis length (0: generic kernel)
     unsigned line_extent = 0;
+    bool line_tma = false;  // TMA-fed (y: from maps)
     int wave_K = 0;   // t: the plane-wave kernel's cluster size (wave_pass.cu; 0: pass by pass)
     int wave_nsample = 0;
     void *ph_steps = nullptr;  // its exp(i dk z) per t-pass (corrected physics)
@@ -615,8 +616,9 @@ void default_variant(const OpoParams &p, int kind, opo::PassVariant &v, size_t &
 // and geometry replace the generic ones.  The bodies measured faster than every generic
 // and warp-specialised variant at each compiled length.  They address a plane with 32-bit
 // byte offsets.
-template <typename C> void use_axis_line(const OpoParams &p, bool xa, PassCfg &pc, std::vector<cd> &tw)
+template <typename C> void use_axis_line(const OpoSolver *s, bool xa, PassCfg &pc, std::vector<cd> &tw)
 {
+    const OpoParams &p = s->p;
     const int n = xa ? p.nx : p.ny;
     if (!opo::axis_line_radix(xa, n, 0) || (size_t)p.nx * p.ny * sizeof(C) > 0xffffffffull) return;
     std::vector<int> rad = {opo::axis_line_radix(xa, n, 0), opo::axis_line_radix(xa, n, 1)};
@@ -640,6 +642,15 @@ template <typename C> void use_axis_line(const OpoParams &p, bool xa, PassCfg &p
     g.gs_j = xa ? 1u : (unsigned)p.nx;
     g.gs_l = xa ? (unsigned)p.nx : 1u;
     pc.smem = xa ? opo::axis_line_smem<C, true>(n) : opo::axis_line_smem<C, false>(n);
+    // TMA-fed where a thread takes one first-stage item and rows are multiples of 16 bytes
+    // (x lines always are); a batch's kernels load through registers
+    pc.line_tma = !s->batched && (xa ? opo::axis_line_tma<C, true>(n)
+                                     : opo::axis_line_tma<C, false>(n) && (size_t)p.nx * sizeof(C) % 16 == 0);
+    if (pc.line_tma && !xa)
+        for (int f = 0; f < 3; f++)
+            pc.line_tma = pc.line_tma && encode_field_map(&pc.maps[f], s->field[f + 1], p.nx, p.ny, p.nt, sizeof(C),
+                                                          L * (unsigned)(sizeof(C) / 8), (unsigned)n, 1);
+    if (pc.line_tma) pc.smem += 16;  // the mbarrier
 }
 
 // Whether the t-pass of setting v runs a line body on this grid.
@@ -868,7 +879,7 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
             }
         }
     }
-    if (kind != kT && !ws) use_axis_line<C>(s->p, kind == kX, pc, tw);
+    if (kind != kT && !ws) use_axis_line<C>(s, kind == kX, pc, tw);
     if (line) {
         if (!use_tpass_line<C>(p, pc, tw)) return fail(s, OPO_ERR_INVALID, "line-specialised t-pass plan");
         if (form) pc.te = (size_t)nt * opo::line_pixels(fp64);
@@ -1201,8 +1212,10 @@ template <typename C> int enqueue_axis(OpoSolver *s, int kind, int which_tab, un
                "axis-pass launch");
     } else if (pc.line_n) {
         const bool square = s->p.nx == s->p.ny;
-        const cudaError_t e = kind == kX ? opo::launch_axis_line_t<C, true>(a, square, pc.smem, s->stream)
-                                         : opo::launch_axis_line_t<C, false>(a, square, pc.smem, s->stream);
+        const CUtensorMap *maps = pc.line_tma ? pc.maps : nullptr;
+        const cudaError_t e = kind == kX
+                                  ? opo::launch_axis_line_t<C, true>(a, square, maps, s->err_dev, pc.smem, s->stream)
+                                  : opo::launch_axis_line_t<C, false>(a, square, maps, s->err_dev, pc.smem, s->stream);
         OPO_CU(s, e, "axis-pass launch");
     } else {
         OPO_CU(s, opo::launch_axis<C>(a, pc.v, kind == kX, pc.grid, pc.smem, s->stream), "axis-pass launch");

@@ -264,8 +264,11 @@ template <typename C> cudaError_t launch_axis(const AxisArgs<C> &a, PassVariant 
 // Line-specialised axis pass (axis_line.cuh) of the fields in a.tmask; square: nx == ny (the
 // y-pass then compiles its row stride in).  configure_axis_line allows its kernels the full
 // shared memory.
+// maps: TMA-fed, y from these tensor maps of the three fields (x ignores them); null: loads
+// through registers.  err: error word of the TMA waits.
 template <typename C, bool X>
-cudaError_t launch_axis_line_t(const AxisArgs<C> &a, bool square, size_t smem, cudaStream_t st);
+cudaError_t launch_axis_line_t(const AxisArgs<C> &a, bool square, const CUtensorMap *maps, int *err, size_t smem,
+                               cudaStream_t st);
 template <typename C, bool X> cudaError_t configure_axis_line_t(int n);
 // Batched form: the kernel over the line tiles of every instance, its CTA size in threads.
 template <typename C, bool X> const void *axis_line_batch_func(int *threads);
