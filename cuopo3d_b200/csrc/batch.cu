@@ -165,7 +165,7 @@ template <typename C> bool batch_t_funcs(PassVariant v, const void *fn[kTGroups]
 {
     for (int g = 0; g < kTGroups - 1; g++) {
         fn[g] = tpass_line_batch_func<C>(kLineNT[g]);
-        threads[g] = tpass_line_shape(kLineNT[g]).threads;
+        threads[g] = tpass_line_shape(sizeof(C) == 16, kLineNT[g]).threads;
     }
     threads[kTGroups - 1] = v.threads;
     if (!is_line(v)) return batch_t_generic_func<C>(v, &fn[kTGroups - 1]);

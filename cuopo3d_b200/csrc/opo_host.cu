@@ -657,7 +657,7 @@ template <typename C> void use_axis_line(const OpoSolver *s, bool xa, PassCfg &p
 template <typename C> bool tpass_line_body(const OpoParams &p, opo::PassVariant v)
 {
     const bool fp64 = sizeof(C) == 16;
-    const opo::LineShape sh = opo::tpass_line_shape(p.nt);
+    const opo::LineShape sh = opo::tpass_line_shape(sizeof(C) == 16, p.nt);
     if (opo::is_ws(v) || (p.flags & OPO_ASIS_Q2) || !sh.ra) return false;
     if ((size_t)p.nx * p.ny % (sh.pp * (fp64 ? 1 : 2))) return false;  // whole tiles only
     return !opo::line_setting_only(p.nt) || (opo::is_line(v) && p.nx % opo::line_pixels(fp64) == 0);
@@ -666,7 +666,7 @@ template <typename C> bool tpass_line_body(const OpoParams &p, opo::PassVariant 
 // The line body's plan and geometry in place of the generic ones.
 template <typename C> bool use_tpass_line(const OpoParams &p, PassCfg &pc, std::vector<cd> &tw)
 {
-    const opo::LineShape sh = opo::tpass_line_shape(p.nt);
+    const opo::LineShape sh = opo::tpass_line_shape(sizeof(C) == 16, p.nt);
     std::vector<int> rad = {sh.ra, sh.rb};
     if (sh.rc > 1) rad.push_back(sh.rc);
     if (!plan_of_radices(p.nt, rad, pc.plan, tw)) return false;
@@ -1546,11 +1546,12 @@ template <typename C> int autotune(OpoSolver *s)
         best.te[kind] = s->pass[kind].te;
         if (kind != kT && !(s->p.flags & OPO_DIFFRACTION)) continue;
         {
-            // a body that runs whatever the classic setting, or the plane-wave kernel: nothing
-            // to time
+            // a compiled body or the plane-wave kernel: ahead of every generic and warp-specialised
+            // variant on its grids, nothing to time
             const opo::PassVariant lv{128, (fp64 ? 4 : 16) | opo::kLineForm};
-            bool line = kind == kT && wave_setting(s, lv) && configure_pass<C>(s, kind, lv, tes[1]) == OPO_OK &&
-                        s->pass[kind].wave_K;
+            bool line = kind == kT && (wave_setting(s, lv) || opo::line_setting_only(s->p.nt)) &&
+                        configure_pass<C>(s, kind, lv, tes[1]) == OPO_OK &&
+                        (s->pass[kind].wave_K || s->pass[kind].line_nt);
             for (int r1 : {8, 4})
                 if (!line && configure_pass<C>(s, kind, opo::PassVariant{128, r1}, tes[1]) == OPO_OK)
                     line = (s->pass[kind].line_n || s->pass[kind].line_nt) && s->pass[kind].v.r1 == r1;
@@ -1575,22 +1576,6 @@ template <typename C> int autotune(OpoSolver *s)
                         best.te[kind] = te;
                     }
                 }
-        // the line setting, where the grid has a body that only it runs
-        for (int r1 : r1s) {
-            const opo::PassVariant lv{128, r1 | opo::kLineForm};
-            // one candidate per precision: its fallback radix (FP32 16, FP64 4) only matters
-            // on grids without a line body
-            if (kind != kT || !opo::variant_compiled(fp64, true, lv) || r1 != (fp64 ? 4 : 16)) continue;
-            if (configure_pass<C>(s, kind, lv, tes[0]) != OPO_OK || !s->pass[kind].line_nt) continue;
-            float ms = 0;
-            int rc = time_pass<C>(s, kind, &ms);
-            if (rc) return rc;
-            if (ms < best_ms) {
-                best_ms = ms;
-                best.v[kind] = s->pass[kind].v;
-                best.te[kind] = tes[0];
-            }
-        }
         int rc = configure_pass<C>(s, kind, best.v[kind], best.te[kind]);
         if (rc) return rc;
     }
@@ -1599,11 +1584,12 @@ template <typename C> int autotune(OpoSolver *s)
         int rc = configure_plane<C>(s, 0, 256, 8);
         if (rc) return rc;
         float best_ms = 1e30f;
-        if ((rc = time_diffraction<C>(s, &best_ms))) return rc;
+        const bool lines = s->pass[kX].line_n && s->pass[kY].line_n;  // ahead of every plane pass
+        if (!lines && (rc = time_diffraction<C>(s, &best_ms))) return rc;
         for (int K : {2, 4, 8})
             for (int th : {256, 512})
                 for (int r1 : r1s) {
-                    if (configure_plane<C>(s, K, th, r1) != OPO_OK) continue;
+                    if (lines || configure_plane<C>(s, K, th, r1) != OPO_OK) continue;
                     if (s->plane.r1 != r1) continue;  // plan fell back to a smaller radix
                     float ms = 0;
                     if ((rc = time_diffraction<C>(s, &ms))) return rc;

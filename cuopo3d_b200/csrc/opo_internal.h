@@ -181,12 +181,12 @@ inline int line_fallback_radix(bool fp64, PassVariant v) { return fp64 ? 4 : rad
 #define OPO_TPASS_LINES(X)                                                                         \
     X(32) X(36) X(48) X(72) X(96) X(108) X(144) X(192) X(216) X(288) X(384) X(432) X(512) X(576)    \
     X(768) X(864) X(1024)
-// Radices (rc = 1: two stages), 16-byte units per time sample, CTA size and CTAs per SM of a
-// line body (tpass_line.cuh); ra = 0: none.
+// Radices (rc = 1: two stages), 16-byte units per time sample, CTA size, CTAs per SM and
+// (stage, field) jobs at a time of a line body (tpass_line.cuh); ra = 0: none.
 struct LineShape {
-    int ra, rb, rc, pp, threads, ctas;
+    int ra, rb, rc, pp, threads, ctas, jobs = 2;
 };
-__host__ __device__ constexpr LineShape tpass_line_shape(int nt)
+__host__ __device__ constexpr LineShape tpass_line_shape(bool fp64, int nt)
 {
     switch (nt) {
     case 32: return {8, 4, 1, 8, 64, 8};
@@ -196,15 +196,15 @@ __host__ __device__ constexpr LineShape tpass_line_shape(int nt)
     case 72: return {9, 8, 1, 8, 192, 3};
     case 96: return {12, 8, 1, 8, 128, 4};
     case 108: return {9, 12, 1, 8, 192, 3};
-    case 128: return {16, 8, 1, 8, 128, 4};
+    case 128: return fp64 ? LineShape{16, 8, 1, 8, 128, 4} : LineShape{16, 8, 1, 8, 192, 4, 3};
     case 144: return {12, 12, 1, 8, 192, 3};
     case 192: return {16, 12, 1, 4, 128, 4};
     case 216: return {9, 6, 4, 4, 192, 3};
     case 256: return {16, 16, 1, 4, 128, 4};
     case 288: return {6, 6, 8, 4, 192, 3};
-    case 384: return {8, 6, 8, 4, 256, 2};
+    case 384: return {6, 8, 8, 4, 384, 2, 3};
     case 432: return {9, 6, 8, 4, 256, 2};
-    case 512: return {8, 8, 8, 4, 256, 2};
+    case 512: return {8, 8, 8, 4, 384, 2, 3};
     case 576: return {9, 8, 8, 2, 192, 3};
     case 768: return {12, 8, 8, 2, 256, 2};
     case 864: return {12, 9, 8, 2, 256, 2};

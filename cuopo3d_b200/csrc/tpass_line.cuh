@@ -17,9 +17,12 @@
 // phase tables are the host's tables of that plan.
 //
 // Shapes (tpass_line_shape): PP and the CTA size give each stage about one item per thread of
-// half a CTA (two (stage, field) jobs run at a time) and 12-18 warps per SM beside tiles
-// of 20-110 KB.  The pass is bound by its arithmetic pipes and by latency (128 x 128 x 256:
-// FP32 FMA pipe 61 %, FP64 pipe 65 % busy), so warps per SM and whole warps per stage decide.
+// half or a third of a CTA (two or three (stage, field) jobs run at a time) and 12-24 warps
+// per SM beside tiles of 20-110 KB.  The pass is bound by its arithmetic pipes and shared
+// memory together (128 x 128 x 256: FP32 FMA pipe 61 %, FP64 pipe 65 % busy): 512 samples took
+// 167-170 us in FP32 with 16, 24 or 32 warps per SM, 256 samples were slower with three jobs
+// (76 against 70 us, register spills) or radix 8 throughout (80 us); three jobs won by 9 % on
+// 64 x 64 x 128 in FP32 (18.4 -> 16.8 us) and by 1-4 % at 384 and 512.
 //
 // Shared memory per field: NT rows of PP units.  With PP < 8 the last stage's threads, RL
 // rows apart, would share banks: two-stage bodies put a padding row after every RL rows,
@@ -326,8 +329,8 @@ template <> struct LineUnit<double2> {
 
 template <typename C, int NT_> struct LineGeom {
     static constexpr int NT = NT_;
-    static constexpr LineShape S = tpass_line_shape(NT);
-    static constexpr int RA = S.ra, RB = S.rb, RC = S.rc, PP = S.pp, THREADS = S.threads, MINB = S.ctas;
+    static constexpr LineShape S = tpass_line_shape(sizeof(C) == 16, NT);
+    static constexpr int RA = S.ra, RB = S.rb, RC = S.rc, PP = S.pp, THREADS = S.threads, MINB = S.ctas, JOBS = S.jobs;
     static constexpr int PX = LineUnit<C>::PX;
     static constexpr int P = PP * PX;            // pixels per tile
     static constexpr int Q = NT / RA;            // butterflies per line of the first stage
@@ -400,8 +403,9 @@ __device__ __forceinline__ void line_sweep(const TPassArgs<C> &a, unsigned base,
         }
     };
     constexpr unsigned NI = G::NT * G::PP;
-    for (unsigned e = threadIdx.x; e < NI; e += 2 * THREADS) {
-        const bool two = e + THREADS < NI;
+    constexpr unsigned PER = 65536 / (G::THREADS * G::MINB) > 100 ? 2 : 1;
+    for (unsigned e = threadIdx.x; e < NI; e += PER * THREADS) {
+        const bool two = PER == 2 && e + THREADS < NI;
         U v0[3], v1[3];
         load(e, v0);
         if (two) load(e + THREADS, v1);
@@ -513,10 +517,9 @@ __device__ __forceinline__ void line_stage_c(const unsigned char *tws_, const un
 }
 
 // The transform stages of every field in tmask as jobs (stage, field) in stage-major
-// order, two jobs per phase (half the CTA each; one job when one field is transformed)
-// and a CTA barrier between phases.  A job's stage of a field always ran in an earlier
-// phase (nf >= 2 jobs apart), and three fields take ceil(3 stages / 2) phases of whole
-// warps instead of one round per stage that leaves half the warps idle for its second half.
+// order, two or three jobs per phase (PER; an equal share of the CTA each; one job when one
+// field is transformed) and a CTA barrier between phases.  A job's stage of a field always
+// ran in an earlier phase (nf >= PER jobs apart).
 template <typename C, typename G, int BAR, int PER>
 __device__ __forceinline__ void line_jobs(const TPassArgs<C> &a, unsigned base, unsigned tmask, unsigned nf, unsigned char *buf)
 {
@@ -569,7 +572,9 @@ __device__ __forceinline__ void tpass_line_tile(const TPassArgs<C> &a, unsigned 
     tile_sync<BAR>();
     if (!tmask) return;
     const unsigned nf = __popc(tmask);
-    if (nf >= 2)
+    if (G::JOBS == 3 && nf == 3)
+        line_jobs<C, G, BAR, G::JOBS>(a, base, tmask, nf, buf);
+    else if (nf >= 2)
         line_jobs<C, G, BAR, 2>(a, base, tmask, nf, buf);
     else
         line_jobs<C, G, BAR, 1>(a, base, tmask, nf, buf);

@@ -114,7 +114,7 @@ template <typename C> cudaError_t launch_tpass_line(const TPassArgs<C> &a, int n
     const void *fn = tpass_line_func<C>(nt, false);
     if (!fn) return cudaErrorInvalidValue;
     void *args[] = {const_cast<TPassArgs<C> *>(&a)};
-    return cudaLaunchKernel(fn, dim3(grid), dim3(tpass_line_shape(nt).threads), args, smem, st);
+    return cudaLaunchKernel(fn, dim3(grid), dim3(tpass_line_shape(sizeof(C) == 16, nt).threads), args, smem, st);
 }
 
 template <typename C>
