@@ -1,6 +1,6 @@
-// Batched line-specialised x- and y-passes: one persistent kernel per precision and axis
-// over the tiles (one field each) of every instance whose axis length has a compiled body;
-// the instance's length selects the body (axis_line.cuh).
+// Batched line-specialised x- and y-passes: one kernel per precision and axis, a CTA per tile
+// (one field each) of every instance whose axis length has a compiled body; the instance's
+// length selects the body (axis_line.cuh).
 #include "axis_line.cuh"
 #include "batch_device.cuh"
 
@@ -15,39 +15,29 @@ __global__ void __launch_bounds__(kBatchThreads<C>, sizeof(C) == 16 ? 8 : 6)
     axis_line_batch_kernel(const AxisArgs<C> *descs, const unsigned *prefix, const BatchHeader *hdr)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    AxisArgs<C> *d = reinterpret_cast<AxisArgs<C> *>(smem_raw);
-    C *sm = reinterpret_cast<C *>(smem_raw + desc_bytes<AxisArgs<C>>());
-    const unsigned ninst = hdr->ninst, total = hdr->total_tiles;
-    descs += hdr->first;
+    C *sm = reinterpret_cast<C *>(smem_raw);
+    const unsigned gt = blockIdx.x;
+    if (gt >= hdr->total_tiles) return;
     prefix += hdr->pfirst;
-    int cur = -1;
-    for (unsigned gt = blockIdx.x; gt < total; gt += gridDim.x) {
-        const int i = find_inst(prefix, ninst, gt);
-        __syncthreads();  // the last tile's shared memory, and the descriptor, are free
-        if (i != cur) {
-            stage_desc(descs + i, d);
-            __syncthreads();
-            cur = i;
-        }
-        unsigned tile = gt - __ldg(prefix + i), f = 0;
-        const unsigned nt = (unsigned)d->g.ntiles;
-        while (tile >= nt) {
-            tile -= nt;
-            f++;
-        }
-        if (!(d->tmask >> f & 1u)) continue;
-        unsigned lim;
-        const unsigned base = axis_line_base(d->g, tile, d->line_extent, lim);
-        switch (d->line_n) {
+    const int i = find_inst(prefix, hdr->ninst, gt);
+    const AxisArgs<C> &d = descs[hdr->first + i];
+    unsigned tile = gt - __ldg(prefix + i), f = 0;
+    const unsigned nt = (unsigned)d.g.ntiles;
+    while (tile >= nt) {
+        tile -= nt;
+        f++;
+    }
+    if (!(d.tmask >> f & 1u)) return;
+    unsigned lim;
+    const unsigned base = axis_line_base(d.g, tile, d.line_extent, lim);
+    switch (d.line_n) {
 #define OPO_CASE(N)                                                                                 \
     case N:                                                                                         \
-        axis_line_tile<C, AxisLine<C, X, N>, kBatchThreads<C>, 0u>(d->f[f] + base, lim, d->g.gs_j, d->tab[f], d->tw, \
-                                                                   sm);                             \
+        axis_line_tile<C, AxisLine<C, X, N>, kBatchThreads<C>, 0u>(d.f[f] + base, lim, d.g.gs_j, d.tab[f], d.tw, sm); \
         break;
-            OPO_AXIS_LINES(OPO_CASE)
+        OPO_AXIS_LINES(OPO_CASE)
 #undef OPO_CASE
-        default: break;
-        }
+    default: break;
     }
 }
 

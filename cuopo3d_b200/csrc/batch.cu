@@ -36,19 +36,17 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 4 : 1)
     const unsigned ninst = hdr->ninst, total = hdr->total_tiles;
     descs += hdr->first;
     prefix += hdr->pfirst;
-    int cur = -1;
+    InstWalk w;
     for (unsigned gt = blockIdx.x; gt < total; gt += gridDim.x) {
-        const int i = find_inst(prefix, ninst, gt);
-        if (i != cur) {
+        if (w.seek(prefix, ninst, gt)) {
             __syncthreads();
-            stage_desc(descs + i, d);
+            stage_desc(descs + w.cur, d);
             __syncthreads();
             if (threadIdx.x < 6 && d->ph_steps) d->ph[threadIdx.x / 3][threadIdx.x % 3] = d->ph_steps[tp * 6 + threadIdx.x];
             __syncthreads();
-            cur = i;
         }
         // stage the tile with cp.async first, as the single-instance t-pass does
-        const unsigned tile = gt - __ldg(prefix + i);
+        const unsigned tile = gt - w.begin;
         const C *src[3] = {d->psrc, d->f[1], d->f[2]};
         stage_tile<C, THREADS, false>(d->g, (unsigned)d->plan.n, tile, src, tpass_load_mask(*d), sm);
         tpass_tile<C, R1, THREADS, RMAX, true>(*d, tile, sm);
@@ -65,16 +63,14 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 4 : 1)
     const unsigned ninst = hdr->ninst, total = hdr->total_tiles;
     descs += hdr->first;
     prefix += hdr->pfirst;
-    int cur = -1;
+    InstWalk w;
     for (unsigned gt = blockIdx.x; gt < total; gt += gridDim.x) {
-        const int i = find_inst(prefix, ninst, gt);
-        if (i != cur) {
+        if (w.seek(prefix, ninst, gt)) {
             __syncthreads();
-            stage_desc(descs + i, d);
+            stage_desc(descs + w.cur, d);
             __syncthreads();
-            cur = i;
         }
-        axis_tile<C, R1, BFAST, THREADS, RMAX>(*d, gt - __ldg(prefix + i), sm);
+        axis_tile<C, R1, BFAST, THREADS, RMAX>(*d, gt - w.begin, sm);
     }
 }
 
@@ -347,6 +343,8 @@ struct OpoBatch {
     // graph was built are not in it: their first instance rebuilds it)
     struct Group {
         bool on = false;
+        bool per_tile = false;  // a line body's: a CTA per tile; else persistent CTAs
+        unsigned tiles = 0;     // per_tile: tiles the graph covers
         int grid = 0;
         size_t smem = 0;  // the largest tile of the group's instances
     };
@@ -554,17 +552,26 @@ template <typename C> int enqueue_batch_round_trip(OpoBatch *b)
     return OPO_OK;
 }
 
-// Whether the graph covers the resident instances: their groups, and their tiles' shared
-// memory.  With grow, the group configuration is extended to what they need.
+// Whether the graph covers the resident instances: their groups, their tiles' shared
+// memory, and the line bodies' tiles.  With grow, the group configuration is extended to
+// what they need, tiles by a quarter at least (a graph is rebuilt in about a millisecond;
+// CTAs past the tiles return at once).
 bool graph_covers(OpoBatch *b, bool grow)
 {
     bool ok = true;
+    unsigned t_tiles[opo::kTGroups] = {}, ax_tiles[2] = {};
     auto need = [&](OpoBatch::Group &g, size_t smem) {
         if (g.on && smem <= g.smem) return;
         ok = false;
         if (!grow) return;
         g.on = true;
         g.smem = std::max(g.smem, smem);
+    };
+    auto need_tiles = [&](OpoBatch::Group &g, unsigned tiles) {
+        g.per_tile = true;
+        if (tiles <= g.tiles) return;
+        ok = false;
+        if (grow) g.tiles = g.tiles ? std::max(tiles, g.tiles + g.tiles / 4) : tiles;
     };
     for (int sidx : b->order) {
         const OpoSolver *s = b->slots[sidx].s;
@@ -575,12 +582,18 @@ bool graph_covers(OpoBatch *b, bool grow)
                                                    : opo::desc_bytes<opo::TPassArgs<float2>>();
         const size_t da = b->precision == OPO_FP64 ? opo::desc_bytes<opo::AxisArgs<double2>>()
                                                    : opo::desc_bytes<opo::AxisArgs<float2>>();
-        need(b->t_group[opo::t_group(opo::solver_line_nt(s))], dt + sm);
+        const int tg = opo::t_group(opo::solver_line_nt(s));
+        need(b->t_group[tg], dt + sm);
+        t_tiles[tg] += (unsigned)nt;
         for (int a = 0; a < 2; a++) {
+            const int ag = ax_group_of(s, 1 + a);
             opo::solver_pass_info(s, 1 + a, &nt, &sm);
-            need(b->ax_group[a][ax_group_of(s, 1 + a)], da + sm);
+            need(b->ax_group[a][ag], ag == 0 ? sm : da + sm);
+            if (ag == 0) ax_tiles[a] += (unsigned)nt;
         }
     }
+    for (int g = 0; g < opo::kTGroups - 1; g++) need_tiles(b->t_group[g], t_tiles[g]);
+    for (int a = 0; a < 2; a++) need_tiles(b->ax_group[a][0], ax_tiles[a]);
     return ok;
 }
 
@@ -597,7 +610,7 @@ template <typename C> int build_batch_graph(OpoBatch *b)
         if (!g.on) return OPO_OK;
         if (g.smem > 227 * 1024) return bfail(b, OPO_ERR_INVALID, "batched tile does not fit in shared memory");
         OPO_BCU(b, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024), "attribute");
-        g.grid = persistent_grid(b, fn, threads, g.smem);
+        g.grid = g.per_tile ? (int)g.tiles : persistent_grid(b, fn, threads, g.smem);
         return OPO_OK;
     };
     for (int g = 0; g < opo::kTGroups; g++)

@@ -36,4 +36,20 @@ __device__ __forceinline__ int find_inst(const unsigned *prefix, unsigned ninst,
     return lo;
 }
 
+// The instance of the ascending tile numbers a persistent CTA walks: its tiles [begin, end)
+// are kept, so a tile of the same instance costs one comparison.
+struct InstWalk {
+    int cur = -1;
+    unsigned begin = 0, end = 0;
+    // Moves to the instance of tile gt; true when it is another one.
+    __device__ __forceinline__ bool seek(const unsigned *prefix, unsigned ninst, unsigned gt)
+    {
+        if (gt < end) return false;
+        cur = find_inst(prefix, ninst, gt);
+        begin = __ldg(prefix + cur);
+        end = __ldg(prefix + cur + 1);
+        return true;
+    }
+};
+
 }  // namespace opo
