@@ -1128,10 +1128,6 @@ TPassArgs<C> make_tpass_args(OpoSolver *s, bool reset_pump, int n_rk4, const dou
     a.n_rk4 = n_rk4;
     const bool phys = (p.flags & OPO_PHYSICS) != 0;
     const double h = 0.5 * p.dz;
-    for (int f = 0; f < 3; f++) a.kappa[f] = (T)p.kappa[f];
-    a.c1 = (T)(phys ? 0.5 * h : 0.5);
-    a.c3 = (T)(phys ? h : 1.0);
-    a.h6 = (T)(h / 6.0);
     for (int f = 0; f < 3; f++) {
         a.c1k[f] = (T)((phys ? 0.5 * h : 0.5) * p.kappa[f]);
         a.c3k[f] = (T)((phys ? h : 1.0) * p.kappa[f]);

@@ -81,9 +81,8 @@ template <typename C> struct TPassArgs {
     unsigned tmask;     // fields that get the t-axis transform
     int n_rk4;          // coupled-wave half steps before the transform (0, 1, 2)
     int use_phase;      // apply exp(-/+ i dk z) (corrected physics)
-    T kappa[3];
-    T c1, c3, h6;       // RK4 stage offsets (k1, k2 -> c1; k3 -> c3) and final weight h/6
-    T c1k[3], c3k[3], h6k[3];  // the same times kappa of each field
+    T c1k[3], c3k[3], h6k[3];  // RK4 stage offsets (k1, k2 -> c1; k3 -> c3) and final weight
+                               // h/6, times kappa of each field
     C ph[2][3];         // exp(i dk z) at the stage positions z, z+h/2, z+h of each half step
     const C *ph_steps;  // batched passes: the ph values of every t-pass of a round trip, [tp][2][3]
     int skip_rows;      // shipped quirk: transform only row y = 0 (tiles with y != 0 skip)

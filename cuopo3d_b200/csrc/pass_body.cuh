@@ -311,36 +311,24 @@ __device__ __forceinline__ void final_stage(C *sm, const TileGeom &g, unsigned n
 // k4 = f(A + c3 k3), A += (k1 + 2 k2 + 2 k3 + k4) h / 6.  The shipped stage offsets are
 // c1 = 0.5, c3 = 1 (no step size); corrected physics uses c1 = h/2, c3 = h.
 
-template <typename C, typename T>
-__device__ __forceinline__ void cwe_rhs(const T *kap, C p, C s, C i, C &dp, C &ds, C &di)
-{
-    C si = cmul(s, i), pic = cmulc(p, i), psc = cmulc(p, s);
-    dp = C{-kap[0] * si.y, kap[0] * si.x};
-    ds = C{-kap[1] * pic.y, kap[1] * pic.x};
-    di = C{-kap[2] * psc.y, kap[2] * psc.x};
-}
-
-template <typename C, typename T>
-__device__ __forceinline__ void cwe_rhs_phase(const T *kap, const C &ph, C p, C s, C i, C &dp, C &ds,
-                                              C &di)
-{
-    cwe_rhs(kap, p, s, i, dp, ds, di);
-    dp = cmulc(dp, ph);
-    ds = cmul(ds, ph);
-    di = cmul(di, ph);
-}
-
 // The products u_p = s i, u_s = p i*, u_i = p s* give k = i kappa u, so every use of k
 // (the next stage's A + c k and the final sum) folds kappa and the step weights into
 // precomputed constants: A + c k = (A.x - c kappa u.y, A.y + c kappa u.x), and
 // A += (h/6) kappa i (u1 + 2 u2 + 2 u3 + u4).  The products and their weighted sum are
 // held with their components swapped, w = (u.y, u.x), so that A + c k = A + (-c kappa,
 // c kappa) * w componentwise: one packed f32x2 fused multiply-add in FP32.
+//
+// With a phase mismatch the products enter times e^{-i dk z} (pump) and e^{+i dk z}
+// (signal, idler) at the stage's z, a.ph[h][0..2] = e^{i dk z} at z, z + h/2, z + h: three more
+// complex products a stage, everything else as without.  Against scaling, rotating and
+// summing the four slopes one by one (FP32: voxel by voxel, not in pairs) the t-pass of
+// 128 x 128 x 256 in corrected physics takes 78 instead of 96 us in FP32, 138 instead of 146 in
+// FP64.
 template <typename C> __device__ __forceinline__ C swp(C u) { return C{u.y, u.x}; }
 template <typename C, typename T>
 __device__ __forceinline__ C add_iku_w(C a, T ck, C w)
 {
-    return C{a.x - ck * w.x, a.y + ck * w.y};
+    return C{__fma_rn(-ck, w.x, a.x), __fma_rn(ck, w.y, a.y)};
 }
 template <> __device__ __forceinline__ float2 add_iku_w<float2, float>(float2 a, float ck, float2 w)
 {
@@ -349,27 +337,69 @@ template <> __device__ __forceinline__ float2 add_iku_w<float2, float>(float2 a,
     return f2unpack(d);
 }
 
-template <typename C>
-__device__ __forceinline__ void rk4_half_fast(const TPassArgs<C> &a, C &p, C &s, C &i)
+// The roundings are fixed in the source (each product that feeds a sum an explicit fused
+// multiply-add or a rounded product), so that the single-instance and the batched kernels,
+// which both inline this, agree bit for bit whatever the compiler would contract in either.
+// (FP32 pairs: packed instructions.)
+__device__ __forceinline__ double rn_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float rn_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double rn_mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float rn_mul(float a, float b) { return __fmul_rn(a, b); }
+// a b and a conj(b)
+template <typename C> __device__ __forceinline__ C rn_cmul(C a, C b)
 {
-    using T = typename TPassArgs<C>::T;
-    C up = swp(cmul(s, i)), us = swp(cmulc(p, i)), ui = swp(cmulc(p, s));  // stage 1
+    return C{rn_fma(a.x, b.x, -rn_mul(a.y, b.y)), rn_fma(a.x, b.y, rn_mul(a.y, b.x))};
+}
+template <typename C> __device__ __forceinline__ C rn_cmulc(C a, C b)
+{
+    return C{rn_fma(a.x, b.x, rn_mul(a.y, b.y)), rn_fma(a.y, b.x, -rn_mul(a.x, b.y))};
+}
+// y + 2 x
+__device__ __forceinline__ double2 rn_add2x(double2 x, double2 y)
+{
+    return double2{__fma_rn(2.0, x.x, y.x), __fma_rn(2.0, x.y, y.y)};
+}
+__device__ __forceinline__ float2 rn_add2x(float2 x, float2 y) { return caxpy(2.f, x, y); }
+__device__ __forceinline__ double2 rn_cadd(double2 a, double2 b) { return double2{__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y)}; }
+__device__ __forceinline__ float2 rn_cadd(float2 a, float2 b) { return cadd(a, b); }
+
+template <bool PH, typename C>
+__device__ __forceinline__ void cwe_products(const C &ph, C p, C s, C i, C &up, C &us, C &ui)
+{
+    up = rn_cmul(s, i);
+    us = rn_cmulc(p, i);
+    ui = rn_cmulc(p, s);
+    if constexpr (PH) {
+        up = rn_cmulc(up, ph);
+        us = rn_cmul(us, ph);
+        ui = rn_cmul(ui, ph);
+    }
+    up = swp(up);
+    us = swp(us);
+    ui = swp(ui);
+}
+
+template <bool PH, typename C>
+__device__ __forceinline__ void rk4_half_step(const TPassArgs<C> &a, int h, C &p, C &s, C &i)
+{
+    C up, us, ui;
+    cwe_products<PH>(a.ph[h][0], p, s, i, up, us, ui);  // stage 1
     C Up = up, Us = us, Ui = ui;
     C p2 = add_iku_w(p, a.c1k[0], up), s2 = add_iku_w(s, a.c1k[1], us), i2 = add_iku_w(i, a.c1k[2], ui);
-    up = swp(cmul(s2, i2)); us = swp(cmulc(p2, i2)); ui = swp(cmulc(p2, s2));  // stage 2
-    Up = caxpy(T(2), up, Up);
-    Us = caxpy(T(2), us, Us);
-    Ui = caxpy(T(2), ui, Ui);
+    cwe_products<PH>(a.ph[h][1], p2, s2, i2, up, us, ui);  // stage 2
+    Up = rn_add2x(up, Up);
+    Us = rn_add2x(us, Us);
+    Ui = rn_add2x(ui, Ui);
     p2 = add_iku_w(p, a.c1k[0], up); s2 = add_iku_w(s, a.c1k[1], us); i2 = add_iku_w(i, a.c1k[2], ui);
-    up = swp(cmul(s2, i2)); us = swp(cmulc(p2, i2)); ui = swp(cmulc(p2, s2));  // stage 3
-    Up = caxpy(T(2), up, Up);
-    Us = caxpy(T(2), us, Us);
-    Ui = caxpy(T(2), ui, Ui);
+    cwe_products<PH>(a.ph[h][1], p2, s2, i2, up, us, ui);  // stage 3
+    Up = rn_add2x(up, Up);
+    Us = rn_add2x(us, Us);
+    Ui = rn_add2x(ui, Ui);
     p2 = add_iku_w(p, a.c3k[0], up); s2 = add_iku_w(s, a.c3k[1], us); i2 = add_iku_w(i, a.c3k[2], ui);
-    up = swp(cmul(s2, i2)); us = swp(cmulc(p2, i2)); ui = swp(cmulc(p2, s2));  // stage 4
-    Up = cadd(Up, up);
-    Us = cadd(Us, us);
-    Ui = cadd(Ui, ui);
+    cwe_products<PH>(a.ph[h][2], p2, s2, i2, up, us, ui);  // stage 4
+    Up = rn_cadd(Up, up);
+    Us = rn_cadd(Us, us);
+    Ui = rn_cadd(Ui, ui);
     p = add_iku_w(p, a.h6k[0], Up);
     s = add_iku_w(s, a.h6k[1], Us);
     i = add_iku_w(i, a.h6k[2], Ui);
@@ -380,7 +410,7 @@ __device__ __forceinline__ void rk4_half_fast(const TPassArgs<C> &a, C &p, C &s,
 // imaginary parts): every product and update then serves both voxels with one packed
 // instruction per component, and a complex product costs 5 instead of 8 instructions
 // for the pair.  u = s i, p i*, p s*;  A + c i kappa u  and  A += (h/6) i kappa (u1 + 2 u2 +
-// 2 u3 + u4)  as in rk4_half_fast.
+// 2 u3 + u4)  as in rk4_half_step.
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 x2_mul(f32x2 a, f32x2 b)
 {
@@ -426,14 +456,31 @@ __device__ __forceinline__ void x2_add_iku(const f32x2 *a, f32x2 c, f32x2 nc, co
     d[1] = x2_fma(u[0], c, a[1]);
 }
 
-__device__ __forceinline__ void rk4_half_fast_x2(const TPassArgs<float2> &a, f32x2 (&p)[2], f32x2 (&s)[2],
-                                                 f32x2 (&i)[2])
+template <bool PH>
+__device__ __forceinline__ void cwe_products_x2(float2 ph, const f32x2 (&p)[2], const f32x2 (&s)[2], const f32x2 (&i)[2],
+                                                f32x2 (&up)[2], f32x2 (&us)[2], f32x2 (&ui)[2])
 {
-    const f32x2 two = x2_dup(2.f);
-    f32x2 up[2], us[2], ui[2], Up[2], Us[2], Ui[2], p2[2], s2[2], i2[2];
     x2_cmul<false>(s, i, up);
     x2_cmul<true>(p, i, us);
     x2_cmul<true>(p, s, ui);
+    if constexpr (PH) {
+        const f32x2 e[2] = {x2_dup(ph.x), x2_dup(ph.y)};
+        f32x2 t[2];
+        x2_cmul<true>(up, e, t);
+        up[0] = t[0]; up[1] = t[1];
+        x2_cmul<false>(us, e, t);
+        us[0] = t[0]; us[1] = t[1];
+        x2_cmul<false>(ui, e, t);
+        ui[0] = t[0]; ui[1] = t[1];
+    }
+}
+
+template <bool PH>
+__device__ __forceinline__ void rk4_half_step_x2(const TPassArgs<float2> &a, int h, f32x2 (&p)[2], f32x2 (&s)[2], f32x2 (&i)[2])
+{
+    const f32x2 two = x2_dup(2.f);
+    f32x2 up[2], us[2], ui[2], Up[2], Us[2], Ui[2], p2[2], s2[2], i2[2];
+    cwe_products_x2<PH>(a.ph[h][0], p, s, i, up, us, ui);
 #pragma unroll
     for (int c = 0; c < 2; c++) { Up[c] = up[c]; Us[c] = us[c]; Ui[c] = ui[c]; }
 #pragma unroll
@@ -442,9 +489,7 @@ __device__ __forceinline__ void rk4_half_fast_x2(const TPassArgs<float2> &a, f32
         x2_add_iku(p, x2_dup(ck[0]), x2_dup(-ck[0]), up, p2);
         x2_add_iku(s, x2_dup(ck[1]), x2_dup(-ck[1]), us, s2);
         x2_add_iku(i, x2_dup(ck[2]), x2_dup(-ck[2]), ui, i2);
-        x2_cmul<false>(s2, i2, up);
-        x2_cmul<true>(p2, i2, us);
-        x2_cmul<true>(p2, s2, ui);
+        cwe_products_x2<PH>(a.ph[h][st < 3 ? 1 : 2], p2, s2, i2, up, us, ui);
 #pragma unroll
         for (int c = 0; c < 2; c++) {
             if (st < 3) {
@@ -470,28 +515,13 @@ __device__ __forceinline__ void rk4_half_fast_x2(const TPassArgs<float2> &a, f32
 template <typename C>
 __device__ __forceinline__ void rk4_half(const TPassArgs<C> &a, int h, C &p, C &s, C &i)
 {
-    using T = typename TPassArgs<C>::T;
-    if (!a.use_phase) {
-        rk4_half_fast(a, p, s, i);
-        return;
-    }
-    C k1p, k1s, k1i, k2p, k2s, k2i, k3p, k3s, k3i, k4p, k4s, k4i;
-    const T c1 = a.c1, c3 = a.c3;
-    const C *ph = a.ph[h];
-    cwe_rhs_phase(a.kappa, ph[0], p, s, i, k1p, k1s, k1i);
-    cwe_rhs_phase(a.kappa, ph[1], C{p.x + c1 * k1p.x, p.y + c1 * k1p.y}, C{s.x + c1 * k1s.x, s.y + c1 * k1s.y},
-                  C{i.x + c1 * k1i.x, i.y + c1 * k1i.y}, k2p, k2s, k2i);
-    cwe_rhs_phase(a.kappa, ph[1], C{p.x + c1 * k2p.x, p.y + c1 * k2p.y}, C{s.x + c1 * k2s.x, s.y + c1 * k2s.y},
-                  C{i.x + c1 * k2i.x, i.y + c1 * k2i.y}, k3p, k3s, k3i);
-    cwe_rhs_phase(a.kappa, ph[2], C{p.x + c3 * k3p.x, p.y + c3 * k3p.y}, C{s.x + c3 * k3s.x, s.y + c3 * k3s.y},
-                  C{i.x + c3 * k3i.x, i.y + c3 * k3i.y}, k4p, k4s, k4i);
-    const T w = a.h6;
-    p.x += (k1p.x + T(2) * k2p.x + T(2) * k3p.x + k4p.x) * w;
-    p.y += (k1p.y + T(2) * k2p.y + T(2) * k3p.y + k4p.y) * w;
-    s.x += (k1s.x + T(2) * k2s.x + T(2) * k3s.x + k4s.x) * w;
-    s.y += (k1s.y + T(2) * k2s.y + T(2) * k3s.y + k4s.y) * w;
-    i.x += (k1i.x + T(2) * k2i.x + T(2) * k3i.x + k4i.x) * w;
-    i.y += (k1i.y + T(2) * k2i.y + T(2) * k3i.y + k4i.y) * w;
+    if (a.use_phase) rk4_half_step<true>(a, h, p, s, i);
+    else rk4_half_step<false>(a, h, p, s, i);
+}
+__device__ __forceinline__ void rk4_half_x2(const TPassArgs<float2> &a, int h, f32x2 (&p)[2], f32x2 (&s)[2], f32x2 (&i)[2])
+{
+    if (a.use_phase) rk4_half_step_x2<true>(a, h, p, s, i);
+    else rk4_half_step_x2<false>(a, h, p, s, i);
 }
 
 // Fields a t-pass must read and write: all three when it applies coupled-wave half
@@ -532,7 +562,7 @@ __device__ __forceinline__ void tpass_tile_split(const TPassArgs<C> &a, unsigned
     if constexpr (sizeof(C) == 8) {
         // FP32: two neighbouring pixels (l, l + 1) per item, their values as packed pairs
         // (16-byte shared-memory accesses; one packed instruction per component for both)
-        if (g.pairs && !a.use_phase && (a.n_rk4 > 0 || a.eom || (lmask & ~tmask))) {
+        if (g.pairs && (a.n_rk4 > 0 || a.eom || (lmask & ~tmask))) {
             for (unsigned e = 2 * threadIdx.x; e < n * P; e += 2 * THREADS) {
                 const unsigned j = fdiv(g.nl, e), l = e - j * P;  // time sample j, pixels l, l + 1
                 const unsigned off = l + prow(g, j) * lsj;
@@ -545,7 +575,7 @@ __device__ __forceinline__ void tpass_tile_split(const TPassArgs<C> &a, unsigned
                     v[f][1] = f2pack(float2{q4.y, q4.w});
                 }
                 for (int h = 0; h < a.n_rk4; h++)
-                    rk4_half_fast_x2(reinterpret_cast<const TPassArgs<float2> &>(a), v[0], v[1], v[2]);
+                    rk4_half_x2(reinterpret_cast<const TPassArgs<float2> &>(a), h, v[0], v[1], v[2]);
                 if (a.eom) {
                     const C ev = __ldg(a.eom + j);
                     const f32x2 er = x2_dup(ev.x), ei = x2_dup(ev.y);

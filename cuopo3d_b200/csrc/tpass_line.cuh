@@ -285,29 +285,11 @@ template <> struct LineUnit<float2> {
     // n half steps of every voxel of the units p, s, i
     __device__ __forceinline__ static void rk4(const TPassArgs<float2> &a, U &p, U &s, U &i)
     {
-        if (!a.use_phase) {
-            f32x2 v[3][2] = {{p.r, p.i}, {s.r, s.i}, {i.r, i.i}};
-            for (int h = 0; h < a.n_rk4; h++) rk4_half_fast_x2(a, v[0], v[1], v[2]);
-            p = X2C{v[0][0], v[0][1]};
-            s = X2C{v[1][0], v[1][1]};
-            i = X2C{v[2][0], v[2][1]};
-            return;
-        }
-        // corrected physics with a phase mismatch: per voxel
-        U *u[3] = {&p, &s, &i};
-        float2 w[2][3];
-#pragma unroll
-        for (int f = 0; f < 3; f++) {
-            const float2 re = f2unpack(u[f]->r), im = f2unpack(u[f]->i);
-            w[0][f] = float2{re.x, im.x};
-            w[1][f] = float2{re.y, im.y};
-        }
-        for (int h = 0; h < a.n_rk4; h++) {
-            rk4_half(a, h, w[0][0], w[0][1], w[0][2]);
-            rk4_half(a, h, w[1][0], w[1][1], w[1][2]);
-        }
-#pragma unroll
-        for (int f = 0; f < 3; f++) *u[f] = X2C{f2pack(float2{w[0][f].x, w[1][f].x}), f2pack(float2{w[0][f].y, w[1][f].y})};
+        f32x2 v[3][2] = {{p.r, p.i}, {s.r, s.i}, {i.r, i.i}};
+        for (int h = 0; h < a.n_rk4; h++) rk4_half_x2(a, h, v[0], v[1], v[2]);
+        p = X2C{v[0][0], v[0][1]};
+        s = X2C{v[1][0], v[1][1]};
+        i = X2C{v[2][0], v[2][1]};
     }
 };
 
@@ -323,7 +305,11 @@ template <> struct LineUnit<double2> {
     __device__ __forceinline__ static U zero() { return double2{0.0, 0.0}; }
     __device__ __forceinline__ static void rk4(const TPassArgs<double2> &a, U &p, U &s, U &i)
     {
-        for (int h = 0; h < a.n_rk4; h++) rk4_half(a, h, p, s, i);
+        if (a.use_phase) {
+            for (int h = 0; h < a.n_rk4; h++) rk4_half_step<true>(a, h, p, s, i);
+        } else {
+            for (int h = 0; h < a.n_rk4; h++) rk4_half_step<false>(a, h, p, s, i);
+        }
     }
 };
 

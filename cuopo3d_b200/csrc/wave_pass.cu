@@ -174,8 +174,8 @@ template <typename C, bool CL> __global__ void __launch_bounds__(kThreads, 1) wa
         for (unsigned i = threadIdx.x; i < ns; i += kThreads) {
             C p = at(0, i), s = at(1, i), d = at(2, i);
             for (int h = 0; h < halves; h++) {
-                if (a.use_phase) rk4_half(phased, h, p, s, d);
-                else rk4_half_fast(a, p, s, d);
+                if (a.use_phase) rk4_half_step<true>(phased, h, p, s, d);
+                else rk4_half_step<false>(a, h, p, s, d);
             }
             if (close && w.closing && w.eom) {
                 const C e = __ldg(w.eom + time_of(i));
