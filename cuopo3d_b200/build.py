@@ -13,7 +13,7 @@ LIB = os.path.join(HERE, "libcuopo3d.so")
 OBJDIR = os.path.join(HERE, "_build")
 SOURCES = [os.path.join(HERE, "csrc", f) for f in ("ssfm_kernels.cu", "opo_host.cu", "noalloc_sums.cu", "batch.cu",
                                                              "init_fields.cu", "serve.cpp", "sweep.cpp", "writer.cpp", "plane_pass.cu", "ws_pass.cu", "tpass_line_32.cu", "tpass_line_64.cu", "axis_line_x32.cu", "axis_line_y32.cu", "axis_line_x64.cu",
-                                                                     "axis_line_y64.cu", "wave_pass.cu", "axis_line_batch.cu",
+                                                                     "axis_line_y64.cu", "wave_pass.cu", "axis_line_batch.cu", "axis_plane.cu",
                                                                      "peaks.cu")]
 HEADERS = [os.path.join(HERE, "csrc", f) for f in ("fft_radix.cuh", "fft_gain.h", "opo_internal.h", "pass_body.cuh", "tpass_line.cuh", "tpass_line_kernels.cuh", "axis_line.cuh", "axis_line_kernels.cuh", "batch_device.cuh", "wave_pass.h", "tma_copy.cuh",
                                                    "solver_internal.h")] + [

@@ -75,6 +75,21 @@ __host__ __device__ constexpr int axis_line_lines(bool fp64, bool x, int n)
     return fp64 ? (x && n >= 216 ? 4 : 8) : (n >= 384 || n == 216 || (x && n == 256) ? 8 : 16);
 }
 
+// Square n x n grids with a body that runs x and y in one launch (axis_plane.cu).
+__host__ __device__ constexpr bool axis_plane(bool fp64, int n) { return n <= (fp64 ? 72 : 64); }
+// Whether it is the faster one on this many planes (fields times nt).  Up to 48 points always:
+// us a z-step, one solver / three in turn, two launches -> one: 32 x 32 x 64 FP64 11.7 / 5.8 ->
+// 10.3 / 5.2, 16 x 16 x 32 FP32 10.3 / 3.9 -> 9.0 / 3.3, 48 x 48 x 256 FP64 43.7 / 36.5 -> 42.1 /
+// 31.7.  From 64 points on two planes per SM are needed (64 x 64 x 64 FP64 22.5 -> 23.9 alone;
+// 64 x 64 x 128 40.0 / 28.8 -> 38.9 / 25.9), and in FP32, whose CTAs a plane's six stages keep
+// longer than the x and y tiles, all planes resident at once, four per SM (64 x 64 x 128 25.0 /
+// 16.3 -> 24.4 / 15.4; x 256 41.9 / 32.3 -> 43.5 / 31.2).  FP32 72 and 96 points: alone 5 and 9 %
+// slower at 256 samples, no body.
+inline bool axis_plane_pays(bool fp64, int n, unsigned planes)
+{
+    return axis_plane(fp64, n) && (n <= 48 || (planes >= 2 * 148 && (fp64 || planes <= 4 * 148)));
+}
+
 // Wavefronts of one shared-memory access of an x stage with nb butterflies per line, butterfly
 // b of line l at element l ls + pos(b), consecutive threads on consecutive butterflies, for
 // elements of which `banks` fill a wavefront (16 FP32, 8 FP64), over 16 wavefronts' threads.

@@ -894,6 +894,10 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
         cudaError_t e = kind == kX ? opo::configure_axis_line_t<C, true>(n) : opo::configure_axis_line_t<C, false>(n);
         if (e != cudaSuccess) return cuda_fail(s, e, "configure line-specialised axis pass");
     }
+    if (pc.line_n && nx == ny) {
+        cudaError_t e = opo::configure_axis_plane<C>(n);
+        if (e != cudaSuccess) return cuda_fail(s, e, "configure line-specialised plane pass");
+    }
     TableSet set;
     set.add<C>(tw, &pc.tw);
     const bool phys = (p.flags & OPO_PHYSICS) != 0;
@@ -1251,11 +1255,33 @@ template <typename C> int enqueue_plane(OpoSolver *s, int which_tab, unsigned ma
     return OPO_OK;
 }
 
+template <typename C> int enqueue_axis_plane(OpoSolver *s, int which_tab, unsigned mask)
+{
+    opo::AxisPlaneArgs<C> a{};
+    for (int f = 0; f < 3; f++) {
+        a.f[f] = fld<C>(s, f + 1);
+        a.tabx[f] = tabs<C>(s, kX, which_tab)[f];
+        a.taby[f] = tabs<C>(s, kY, which_tab)[f];
+    }
+    a.twx = static_cast<const C *>(s->pass[kX].tw);
+    a.twy = static_cast<const C *>(s->pass[kY].tw);
+    a.tmask = mask;
+    a.nt = (unsigned)s->p.nt;
+    OPO_CU(s, opo::launch_axis_plane<C>(a, s->p.nx, s->stream), "plane launch");
+    s->launches++;
+    return OPO_OK;
+}
+
 // The diffraction operator of a z-step (which_tab 0) or the free-space return (1) on
-// the fields in mask: one fused plane pass, or the x then the y pass.
+// the fields in mask: one plane pass of clusters, the x then the y pass, or these in one launch.
 template <typename C> int enqueue_diffraction(OpoSolver *s, int which_tab, unsigned mask)
 {
     if (s->plane.K) return enqueue_plane<C>(s, which_tab, mask);
+    // square grids where one launch of both line passes pays; pass timing keeps them apart
+    // (the same results)
+    const int n = s->p.nx == s->p.ny && s->pass[kX].line_n && s->pass[kY].line_n ? s->p.nx : 0;
+    const unsigned planes = (unsigned)__builtin_popcount(mask) * (unsigned)s->p.nt;
+    if (n && !s->timing && opo::axis_plane_pays(sizeof(C) == 16, n, planes)) return enqueue_axis_plane<C>(s, which_tab, mask);
     int rc;
     if ((rc = enqueue_axis<C>(s, kX, which_tab, mask))) return rc;
     return enqueue_axis<C>(s, kY, which_tab, mask);

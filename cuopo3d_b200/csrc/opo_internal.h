@@ -104,6 +104,14 @@ template <typename C> struct AxisArgs {
     unsigned line_extent;  // lines of a tile row (y: nx) or of the field (x: ny nt)
 };
 
+// Both line passes of a square grid, a plane of one field per CTA (axis_plane.cu).
+template <typename C> struct AxisPlaneArgs {
+    C *f[3];
+    const C *twx, *twy;
+    const typename TabOf<C>::type *tabx[3], *taby[3];  // the x- and y-pass's own tables
+    unsigned tmask, nt;
+};
+
 // Fused (x, y) diffraction pass over whole (field, t) planes.  A cluster of K CTAs owns
 // one plane: CTA r first holds rows [r ny/K, (r+1) ny/K) in its slab (x geometry gx:
 // rows of nx + 1 elements) and applies the x factor to them; after a cluster barrier
@@ -269,6 +277,10 @@ template <typename C, bool X>
 cudaError_t launch_axis_line_t(const AxisArgs<C> &a, bool square, const CUtensorMap *maps, int *err, size_t smem,
                                cudaStream_t st);
 template <typename C, bool X> cudaError_t configure_axis_line_t(int n);
+// x then y line pass of a square grid in one launch (axis_plane.cu), n points a side;
+// configure_axis_plane allows its kernel the full shared memory where it needs it.
+template <typename C> cudaError_t launch_axis_plane(const AxisPlaneArgs<C> &a, int n, cudaStream_t st);
+template <typename C> cudaError_t configure_axis_plane(int n);
 // Batched form: the kernel over the line tiles of every instance, its CTA size in threads.
 template <typename C, bool X> const void *axis_line_batch_func(int *threads);
 template <typename C> cudaError_t launch_sums(const C *f0, const C *f1, const C *f2, size_t n,

@@ -231,7 +231,8 @@ int opo_run_round_trips_tallied(OpoSolver *s, int n, double *tallies, int *done)
 
 /* Per-pass device timing with CUDA events on the solver's stream.  While enabled,
  * passes are launched one by one (round trips are not replayed as graphs) with an event
- * pair around every pass kernel.  opo_pass_times() waits for the stream, returns the
+ * pair around every pass kernel, and x and y passes that otherwise share a launch (small
+ * square grids; the results are the same) apart.  opo_pass_times() waits for the stream, returns the
  * accumulated milliseconds and launch counts per pass kind since the last call --
  * [0] t-pass, [1] x-pass or fused (x, y) plane pass, [2] y-pass, [3] other kernels --
  * and resets them.
