@@ -339,6 +339,7 @@ struct OpoBatch {
     bool dirty = true;
     std::vector<char> last_flag;  // per order position: on its last round trip when uploaded
     cudaGraphExec_t graph = nullptr;
+    int graph_steps = 0;  // z-steps of the graph's round trip
     // launch configuration of every group in the graph (groups without instances when the
     // graph was built are not in it: their first instance rebuilds it)
     struct Group {
@@ -552,13 +553,13 @@ template <typename C> int enqueue_batch_round_trip(OpoBatch *b)
     return OPO_OK;
 }
 
-// Whether the graph covers the resident instances: their groups, their tiles' shared
-// memory, and the line bodies' tiles.  With grow, the group configuration is extended to
+// Whether the graph covers the resident instances: their z-steps, their groups, their tiles'
+// shared memory, and the line bodies' tiles.  With grow, the group configuration is extended to
 // what they need, tiles by a quarter at least (a graph is rebuilt in about a millisecond;
 // CTAs past the tiles return at once).
 bool graph_covers(OpoBatch *b, bool grow)
 {
-    bool ok = true;
+    bool ok = b->graph_steps == b->n_steps;
     unsigned t_tiles[opo::kTGroups] = {}, ax_tiles[2] = {};
     auto need = [&](OpoBatch::Group &g, size_t smem) {
         if (g.on && smem <= g.smem) return;
@@ -630,6 +631,7 @@ template <typename C> int build_batch_graph(OpoBatch *b)
     if (e != cudaSuccess) return bfail(b, OPO_ERR_CUDA, std::string("end capture: ") + cudaGetErrorString(e));
     b->launches_rt = (int)(b->launches - before);
     b->launches = before;
+    b->graph_steps = b->n_steps;
     e = cudaGraphInstantiate(&b->graph, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return bfail(b, OPO_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
