@@ -15,7 +15,7 @@ SOURCES = [os.path.join(HERE, "csrc", f) for f in ("ssfm_kernels.cu", "opo_host.
                                                              "init_fields.cu", "serve.cpp", "sweep.cpp", "writer.cpp", "plane_pass.cu", "ws_pass.cu", "tpass_line_32.cu", "tpass_line_64.cu", "axis_line_x32.cu", "axis_line_y32.cu", "axis_line_x64.cu",
                                                                      "axis_line_y64.cu", "wave_pass.cu", "axis_line_batch.cu", "axis_plane.cu",
                                                                      "peaks.cu")]
-HEADERS = [os.path.join(HERE, "csrc", f) for f in ("fft_radix.cuh", "fft_gain.h", "opo_internal.h", "pass_body.cuh", "tpass_line.cuh", "tpass_line_kernels.cuh", "axis_line.cuh", "axis_line_kernels.cuh", "batch_device.cuh", "wave_pass.h", "tma_copy.cuh",
+HEADERS = [os.path.join(HERE, "csrc", f) for f in ("fft_radix.cuh", "fft_gain.h", "opo_internal.h", "pass_body.cuh", "tpass_line.cuh", "tpass_line_kernels.cuh", "axis_line.cuh", "axis_line_kernels.cuh", "batch_device.cuh", "block_arena.h", "wave_pass.h", "tma_copy.cuh",
                                                    "solver_internal.h")] + [
     os.path.join(ROOT, "include", "cuopo3d.h")]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

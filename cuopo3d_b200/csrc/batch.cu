@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "batch_device.cuh"
+#include "block_arena.h"
 #include "pass_body.cuh"
 #include "solver_internal.h"
 
@@ -209,97 +210,28 @@ namespace {
 
 using cd = std::complex<double>;
 
-// Device memory of a batch's instances.  A cudaMalloc / cudaFree pair of an instance's size
-// takes 0.7 ms and the free waits for the device, so blocks come from slabs of up to eight
-// small instances, and a removed instance's block serves the next one of about its size.
-// What is held beyond the resident instances stays within the batch's HBM budget and, idle,
-// within kIdleBytes; the rest goes back to the driver at once, everything with the batch.
-class BlockArena {
-public:
-    // A block of at least `need` bytes; up to `more` further instances may be admitted into
-    // `spare` bytes of budget.  Null: out of memory.
-    void *take(size_t need, int more, size_t spare, size_t budget)
+// The arena's memory (block_arena.h): device memory of the batch's device, copies in the order of
+// its stream.
+struct BatchMem {
+    OpoBatch *b;
+    void *alloc(size_t n)
     {
-        int best = -1;
-        for (int k = 0; k < (int)blocks_.size(); k++) {
-            const Block &b = blocks_[k];
-            // larger blocks only when the budget leaves no room for another slab
-            if (b.used || b.size < need || (b.size > need + need / 4 && held_ + need <= budget)) continue;
-            if (best < 0 || b.size < blocks_[best].size) best = k;
-        }
-        if (best < 0) {
-            size_t n = std::min<size_t>({8, (size_t)more + 1, 1 + spare / need, std::max<size_t>(1, kIdleBytes / need)});
-            if (held_ + n * need > budget) {
-                trim(0);
-                if (held_ + n * need > budget) n = 1;
-            }
-            void *p = nullptr;
-            if (cudaMalloc(&p, n * need) != cudaSuccess) {
-                (void)cudaGetLastError();
-                trim(0);
-                n = 1;
-                if (cudaMalloc(&p, need) != cudaSuccess) return nullptr;
-            }
-            held_ += n * need;
-            best = (int)blocks_.size();
-            for (size_t k = 0; k < n; k++) blocks_.push_back({static_cast<char *>(p) + k * need, need, p, n * need, false});
-        }
-        blocks_[best].used = true;
-        return blocks_[best].p;
+        void *p = nullptr;
+        if (cudaMalloc(&p, n) == cudaSuccess) return p;
+        (void)cudaGetLastError();
+        return nullptr;
     }
-    size_t size_of(const void *p) const
+    void free(void *p) { cudaFree(p); }
+    void *alloc_host(size_t n)
     {
-        for (const Block &b : blocks_)
-            if (b.p == p) return b.size;
-        return 0;
+        void *p = nullptr;
+        if (cudaHostAlloc(&p, n, cudaHostAllocDefault) == cudaSuccess) return p;
+        (void)cudaGetLastError();
+        return nullptr;
     }
-    // The caller has synchronised with the work on the block.
-    void give(const void *p)
-    {
-        for (Block &b : blocks_)
-            if (b.p == p) b.used = false;
-        trim(kIdleBytes);
-    }
-    ~BlockArena()
-    {
-        for (Block &b : blocks_) b.used = false;
-        trim(0);
-    }
-
-private:
-    struct Block {
-        char *p;
-        size_t size;
-        void *slab;
-        size_t slab_bytes;
-        bool used;
-    };
-    static constexpr size_t kIdleBytes = (size_t)256 << 20;
-    // Frees wholly idle slabs while more than `keep` bytes are idle.
-    void trim(size_t keep)
-    {
-        size_t idle = 0;
-        for (const Block &b : blocks_)
-            if (!b.used) idle += b.size;
-        for (size_t k = 0; k < blocks_.size() && idle > keep;) {
-            void *slab = blocks_[k].slab;
-            const size_t bytes = blocks_[k].slab_bytes;
-            bool busy = false;
-            for (const Block &b : blocks_) busy |= b.slab == slab && b.used;
-            if (busy) {
-                k++;
-                continue;
-            }
-            blocks_.erase(std::remove_if(blocks_.begin(), blocks_.end(), [&](const Block &b) { return b.slab == slab; }),
-                          blocks_.end());
-            cudaFree(slab);
-            held_ -= bytes;
-            idle -= bytes;
-            k = 0;
-        }
-    }
-    std::vector<Block> blocks_;
-    size_t held_ = 0;
+    void free_host(void *p) { cudaFreeHost(p); }
+    bool copy(void *to, const void *from, size_t n);
+    void moved(void *from, void *to, size_t n);
 };
 
 struct Slot {
@@ -322,7 +254,7 @@ struct OpoBatch {
     int dev = 0;
     int sms = 148;
     size_t budget = 0, used = 0;
-    BlockArena arena;
+    opo::BlockArena<BatchMem> arena{BatchMem{this}};
     opo::PassVariant v[3];
     size_t te[3];
     cudaStream_t stream = nullptr;
@@ -373,6 +305,24 @@ int bfail(OpoBatch *b, int code, const std::string &msg)
             return bfail((b), e_ == cudaErrorMemoryAllocation ? OPO_ERR_NOMEM : OPO_ERR_CUDA,   \
                          std::string(what) + ": " + cudaGetErrorString(e_));                    \
     } while (0)
+
+bool BatchMem::copy(void *to, const void *from, size_t n)
+{
+    if (cudaMemcpyAsync(to, from, n, cudaMemcpyDefault, b->stream) == cudaSuccess &&
+        cudaStreamSynchronize(b->stream) == cudaSuccess)
+        return true;
+    (void)cudaGetLastError();
+    return false;
+}
+void BatchMem::moved(void *from, void *to, size_t n)
+{
+    for (Slot &sl : b->slots)
+        if (sl.used && sl.block == from) {
+            opo::solver_move_block(sl.s, to, n);
+            sl.block = to;
+            b->dirty = true;
+        }
+}
 
 bool slot_ok(const OpoBatch *b, int slot) { return b && slot >= 0 && slot < b->capacity && b->slots[slot].used; }
 
@@ -791,18 +741,18 @@ int opo_batch_add(OpoBatch *b, const OpoParams *p, const double *w, int *slot_ou
     const size_t need = opo::batch_instance_bytes(b->precision, V);  // fields + tables and plans
     if (b->used + need > b->budget) return bfail(b, OPO_ERR_CAPACITY, "HBM budget exhausted");
     OpoSolver *s = nullptr;
-    void *block = b->arena.take(need, b->capacity - (int)b->order.size() - 1, b->budget - b->used - need, b->budget);
+    void *block = b->arena.take(need, b->capacity - (int)b->order.size() - 1, b->budget);
     if (!block) return bfail(b, OPO_ERR_NOMEM, "instance memory");
-    int rc = opo::solver_create_configured(p, w, b->v, b->te, b->stream, block, b->arena.size_of(block), &s);
+    int rc = opo::solver_create_configured(p, w, b->v, b->te, b->stream, block, need, &s);
     if (rc) {
-        b->arena.give(block);
+        b->arena.give(block, b->budget);
         return bfail(b, rc, "instance creation failed (grid not supported by the batch's kernel variants?)");
     }
     for (int k = 0; k < 3; k++) {
         const opo::PassVariant got = opo::solver_pass_variant(s, k);
         if (got.r1 != b->v[k].r1 || got.threads != b->v[k].threads || (k == 0 && !opo::solver_line_fallback_ok(s))) {
             opo_destroy(s);
-            b->arena.give(block);
+            b->arena.give(block, b->budget);
             return bfail(b, OPO_ERR_INVALID, "grid needs a first-stage radix other than the batch's");
         }
     }
@@ -831,7 +781,7 @@ int opo_batch_add(OpoBatch *b, const OpoParams *p, const double *w, int *slot_ou
         const size_t bytes = ph.size() * esz;
         if (cudaMalloc(&sl.ph_steps, bytes) != cudaSuccess) {
             opo_destroy(s);
-            b->arena.give(block);
+            b->arena.give(block, b->budget);
             sl = Slot{};
             return bfail(b, OPO_ERR_NOMEM, "phase table allocation");
         }
@@ -861,12 +811,13 @@ int opo_batch_remove(OpoBatch *b, int slot)
     Slot &sl = b->slots[slot];
     cudaStreamSynchronize(b->stream);
     opo_destroy(sl.s);
-    b->arena.give(sl.block);
     if (sl.ph_steps) cudaFree(sl.ph_steps);
+    const void *block = sl.block;
     b->used -= sl.bytes;
     sl = Slot{};
     b->order.erase(std::remove(b->order.begin(), b->order.end(), slot), b->order.end());
     b->dirty = true;
+    b->arena.give(block, b->budget);
     return OPO_OK;
 }
 

@@ -2279,6 +2279,36 @@ int solver_create_configured(const OpoParams *p, const double *w, const PassVari
     return create_impl(p, w, v, te, stream, block, block_bytes, out);
 }
 
+void solver_move_block(OpoSolver *s, void *to, size_t block_bytes)
+{
+    char *const from = static_cast<char *>(s->mem);
+    auto move = [&](auto &p) {
+        char *c = (char *)p;
+        if (c >= from && c < from + block_bytes) p = reinterpret_cast<std::decay_t<decltype(p)>>(static_cast<char *>(to) + (c - from));
+    };
+    for (auto &f : s->field) move(f);
+    move(s->partials);
+    move(s->sums_dev);
+    move(s->err_dev);
+    if (s->table_left) move(s->table_area);
+    for (auto &pc : s->pass) {  // (a batch's instance has no tensor maps)
+        move(pc.tw);
+        move(pc.eom);
+        move(pc.ph_steps);
+        for (auto &row : pc.tab)
+            for (auto &t : row) move(t);
+    }
+    move(s->plane.twx);
+    move(s->plane.twy);
+    for (int k = 0; k < 2; k++)
+        for (int f = 0; f < 3; f++) {
+            move(s->plane.tabx[k][f]);
+            move(s->plane.taby[k][f]);
+        }
+    drop_graphs(s);
+    s->mem = to;
+}
+
 PassVariant solver_pass_variant(const OpoSolver *s, int kind) { return s->pass[kind].v; }
 
 bool solver_line_fallback_ok(const OpoSolver *s)

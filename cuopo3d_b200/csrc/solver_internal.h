@@ -22,6 +22,9 @@ inline size_t batch_instance_bytes(int precision, size_t voxels)
 // caller keeps both until the solver is destroyed.
 int solver_create_configured(const OpoParams *p, const double *w, const PassVariant v[3], const size_t te[3],
                              cudaStream_t stream, void *block, size_t block_bytes, OpoSolver **out);
+// The block of a solver created on one has been copied to `to` (block_bytes as then): every
+// address in it follows.
+void solver_move_block(OpoSolver *s, void *to, size_t block_bytes);
 void solver_pass_info(const OpoSolver *s, int kind, int *ntiles, size_t *smem);
 PassVariant solver_pass_variant(const OpoSolver *s, int kind);
 // A line-specialised t-pass setting runs its line body on s's grid, or its generic
