@@ -245,6 +245,24 @@ struct Slot {
     long long voxels = 0;
 };
 
+// Launch configuration of the groups of instances that share a kernel.
+struct BatchGroup {
+    bool on = false;
+    bool per_tile = false;  // a line body's: a CTA per tile; else persistent CTAs
+    unsigned tiles = 0;
+    int grid = 0;
+    size_t smem = 0;  // the largest tile of the group's instances
+};
+struct BatchGroups {
+    BatchGroup t[opo::kTGroups], ax[2][opo::kAxGroups];
+    template <typename F> void each(const BatchGroups &other, F f)
+    {
+        for (int g = 0; g < opo::kTGroups; g++) f(t[g], other.t[g]);
+        for (int a = 0; a < 2; a++)
+            for (int g = 0; g < opo::kAxGroups; g++) f(ax[a][g], other.ax[a][g]);
+    }
+};
+
 }  // namespace
 
 struct OpoBatch {
@@ -272,16 +290,8 @@ struct OpoBatch {
     std::vector<char> last_flag;  // per order position: on its last round trip when uploaded
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0;  // z-steps of the graph's round trip
-    // launch configuration of every group in the graph (groups without instances when the
-    // graph was built are not in it: their first instance rebuilds it)
-    struct Group {
-        bool on = false;
-        bool per_tile = false;  // a line body's: a CTA per tile; else persistent CTAs
-        unsigned tiles = 0;     // per_tile: tiles the graph covers
-        int grid = 0;
-        size_t smem = 0;  // the largest tile of the group's instances
-    };
-    Group t_group[opo::kTGroups], ax_group[2][opo::kAxGroups];
+    BatchGroups groups;   // launch configuration of the graph
+    double carried_us = 0;  // what it carried beyond the instances' needs since it was built
     long long launches = 0;
     int launches_rt = 0;
     std::string err;
@@ -467,12 +477,12 @@ template <typename C> int enqueue_batch_round_trip(OpoBatch *b)
         const TA *descs = static_cast<const TA *>(b->d_t[which]);
         const unsigned *pre = b->d_prefix[0];
         for (int g = 0; g < opo::kTGroups; g++) {
-            if (!b->t_group[g].on) continue;
+            if (!b->groups.t[g].on) continue;
             const opo::BatchHeader *h = hdr + g;
             void *args[] = {(void *)&descs, (void *)&pre, (void *)&h, (void *)&tp};
             b->launches++;
-            cudaError_t e = cudaLaunchKernel(f.t[g], dim3(b->t_group[g].grid), dim3(f.t_threads[g]), args,
-                                             b->t_group[g].smem, b->stream);
+            cudaError_t e = cudaLaunchKernel(f.t[g], dim3(b->groups.t[g].grid), dim3(f.t_threads[g]), args,
+                                             b->groups.t[g].smem, b->stream);
             if (e != cudaSuccess) return e;
         }
         return cudaSuccess;
@@ -481,7 +491,7 @@ template <typename C> int enqueue_batch_round_trip(OpoBatch *b)
         const AA *descs = static_cast<const AA *>(b->d_ax[axis][which]);
         const unsigned *pre = b->d_prefix[1 + axis];
         for (int g = 0; g < opo::kAxGroups; g++) {
-            const OpoBatch::Group &gr = b->ax_group[axis][g];
+            const BatchGroup &gr = b->groups.ax[axis][g];
             if (!gr.on) continue;
             const opo::BatchHeader *h = hdr + opo::kTGroups + axis * opo::kAxGroups + g;
             void *args[] = {(void *)&descs, (void *)&pre, (void *)&h};
@@ -503,61 +513,83 @@ template <typename C> int enqueue_batch_round_trip(OpoBatch *b)
     return OPO_OK;
 }
 
-// Whether the graph covers the resident instances: their z-steps, their groups, their tiles'
-// shared memory, and the line bodies' tiles.  With grow, the group configuration is extended to
-// what they need, tiles by a quarter at least (a graph is rebuilt in about a millisecond;
-// CTAs past the tiles return at once).
-bool graph_covers(OpoBatch *b, bool grow)
+// What the resident instances need of a round trip's launches.
+BatchGroups needed_groups(const OpoBatch *b)
 {
-    bool ok = b->graph_steps == b->n_steps;
-    unsigned t_tiles[opo::kTGroups] = {}, ax_tiles[2] = {};
-    auto need = [&](OpoBatch::Group &g, size_t smem) {
-        if (g.on && smem <= g.smem) return;
-        ok = false;
-        if (!grow) return;
+    BatchGroups need;
+    const size_t dt = b->precision == OPO_FP64 ? opo::desc_bytes<opo::TPassArgs<double2>>()
+                                               : opo::desc_bytes<opo::TPassArgs<float2>>();
+    const size_t da = b->precision == OPO_FP64 ? opo::desc_bytes<opo::AxisArgs<double2>>()
+                                               : opo::desc_bytes<opo::AxisArgs<float2>>();
+    auto take = [](BatchGroup &g, bool per_tile, int tiles, size_t smem) {
         g.on = true;
+        g.per_tile = per_tile;
+        g.tiles += (unsigned)tiles;
         g.smem = std::max(g.smem, smem);
-    };
-    auto need_tiles = [&](OpoBatch::Group &g, unsigned tiles) {
-        g.per_tile = true;
-        if (tiles <= g.tiles) return;
-        ok = false;
-        if (grow) g.tiles = g.tiles ? std::max(tiles, g.tiles + g.tiles / 4) : tiles;
     };
     for (int sidx : b->order) {
         const OpoSolver *s = b->slots[sidx].s;
         int nt;
         size_t sm;
         opo::solver_pass_info(s, 0, &nt, &sm);
-        const size_t dt = b->precision == OPO_FP64 ? opo::desc_bytes<opo::TPassArgs<double2>>()
-                                                   : opo::desc_bytes<opo::TPassArgs<float2>>();
-        const size_t da = b->precision == OPO_FP64 ? opo::desc_bytes<opo::AxisArgs<double2>>()
-                                                   : opo::desc_bytes<opo::AxisArgs<float2>>();
         const int tg = opo::t_group(opo::solver_line_nt(s));
-        need(b->t_group[tg], dt + sm);
-        t_tiles[tg] += (unsigned)nt;
+        take(need.t[tg], tg < opo::kTGroups - 1, nt, dt + sm);
         for (int a = 0; a < 2; a++) {
             const int ag = ax_group_of(s, 1 + a);
             opo::solver_pass_info(s, 1 + a, &nt, &sm);
-            need(b->ax_group[a][ag], ag == 0 ? sm : da + sm);
-            if (ag == 0) ax_tiles[a] += (unsigned)nt;
+            take(need.ax[a][ag], ag == 0, nt, ag == 0 ? sm : da + sm);
         }
     }
-    for (int g = 0; g < opo::kTGroups - 1; g++) need_tiles(b->t_group[g], t_tiles[g]);
-    for (int a = 0; a < 2; a++) need_tiles(b->ax_group[a][0], ax_tiles[a]);
+    return need;
+}
+
+// Whether the graph covers the resident instances: their z-steps, their groups, their tiles'
+// shared memory, and the line bodies' tiles.
+bool graph_covers(OpoBatch *b, const BatchGroups &need)
+{
+    bool ok = b->graph && b->graph_steps == b->n_steps;
+    b->groups.each(need, [&](const BatchGroup &g, const BatchGroup &n) {
+        ok = ok && (!n.on || (g.on && n.smem <= g.smem && (!n.per_tile || n.tiles <= g.tiles)));
+    });
     return ok;
 }
 
-template <typename C> int build_batch_graph(OpoBatch *b)
+// Whether to rebuild a graph that covers more than the resident instances: once what it has
+// carried beyond them costs as much as the new graph.  B200: a launch without instances takes
+// 1 us, a CTA past the tiles 0.5 ns (0.76 with 100 KB of shared memory), a tile whose group
+// has more than twice the shared memory it needs about 1.5 ns longer; a graph is captured,
+// instantiated and first launched in about 3 us per node.
+bool graph_outgrown(OpoBatch *b, const BatchGroups &need)
 {
+    double ns = 0;
+    b->groups.each(need, [&](const BatchGroup &g, const BatchGroup &n) {
+        if (!g.on) return;
+        if (!n.on) ns += 1000;
+        if (g.per_tile) ns += 0.5 * (g.tiles - n.tiles);
+        if (n.on && g.smem > 2 * n.smem) ns += 1.5 * n.tiles;
+    });
+    b->carried_us += 1e-3 * ns * (b->n_steps + 1);
+    return b->carried_us > 3.0 * b->launches_rt;
+}
+
+// Captures the round trip of the resident instances, which need `need`; a line group that
+// outgrew the last graph gets a quarter more tiles than that had at least, so that instances
+// joining one by one do not rebuild it each time.
+template <typename C> int build_batch_graph(OpoBatch *b, const BatchGroups &need)
+{
+    BatchGroups groups = need;
+    groups.each(b->groups, [](BatchGroup &g, const BatchGroup &old) {
+        if (g.per_tile && old.tiles && g.tiles > old.tiles) g.tiles = std::max(g.tiles, old.tiles + old.tiles / 4);
+    });
+    b->groups = BatchGroups{};
+    b->carried_us = 0;
     if (b->graph) {
         cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
     }
-    graph_covers(b, true);
     BatchFuncs<C> f;
     if (!batch_funcs<C>(b, f)) return bfail(b, OPO_ERR_INVALID, "batch kernel variant not compiled");
-    auto configure = [&](OpoBatch::Group &g, const void *fn, int threads) -> int {
+    auto configure = [&](BatchGroup &g, const void *fn, int threads) -> int {
         if (!g.on) return OPO_OK;
         if (g.smem > 227 * 1024) return bfail(b, OPO_ERR_INVALID, "batched tile does not fit in shared memory");
         OPO_BCU(b, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024), "attribute");
@@ -565,10 +597,11 @@ template <typename C> int build_batch_graph(OpoBatch *b)
         return OPO_OK;
     };
     for (int g = 0; g < opo::kTGroups; g++)
-        if (int rc = configure(b->t_group[g], f.t[g], f.t_threads[g])) return rc;
+        if (int rc = configure(groups.t[g], f.t[g], f.t_threads[g])) return rc;
     for (int a = 0; a < 2; a++)
         for (int g = 0; g < opo::kAxGroups; g++)
-            if (int rc = configure(b->ax_group[a][g], f.ax[a][g], f.ax_threads[a][g])) return rc;
+            if (int rc = configure(groups.ax[a][g], f.ax[a][g], f.ax_threads[a][g])) return rc;
+    b->groups = groups;
     cudaGraph_t g = nullptr;
     OPO_BCU(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
     const long long before = b->launches;
@@ -601,8 +634,9 @@ template <typename C> int batch_run(OpoBatch *b, int n)
             int rc = upload_descriptors<C>(b);
             if (rc) return rc;
         }
-        if (!b->graph || !graph_covers(b, false)) {
-            int rc = build_batch_graph<C>(b);
+        const BatchGroups groups = needed_groups(b);
+        if (!graph_covers(b, groups) || graph_outgrown(b, groups)) {
+            int rc = build_batch_graph<C>(b, groups);
             if (rc) return rc;
         }
         OPO_BCU(b, cudaGraphLaunch(b->graph, b->stream), "batch graph launch");
