@@ -1,5 +1,5 @@
-// Gain compensation of the FP32 transform pairs (host code, shared by the solver's
-// table builder and the host-side check in tests/native/gain_check.cu).
+// Gain compensation of the transform pairs (host code, shared by the solver's table builder
+// and the host-side checks in tests/native/gain_check.cu and gain64_check.cu).
 //
 // The FP32 kernels' roots of unity -- the butterflies' constants (fft_radix.cuh) and the
 // stage twiddles, computed in FP64 and rounded -- have |W|^2 - 1 of a few 1e-8, mostly
@@ -13,6 +13,12 @@
 // at spectrum position p gives the pair the energy gain of the table itself for white
 // inputs, which removes the coherent drain.  What remains is the arithmetic's own
 // rounding.
+//
+// FP64 likewise, a factor 2^29 smaller: the double nearest cos(pi/4) is 1 + 6.8e-17 of it, so
+// a pair of radices 8 x 8 multiplies amplitudes by 1 + 6.5e-17 on average where 4 x 4 x 4 leaves
+// 1 + 3e-18, in phase at every step: 1.5e-14 of the power over 120 steps.  The factors are held
+// and applied to the table entries in extended precision; the entries' own rounding to FP64
+// is as large but differs in sign from entry to entry.
 #pragma once
 
 #include "fft_radix.cuh"
@@ -90,7 +96,91 @@ inline std::vector<double> fp32_pair_compensation(const AxisPlan &pl, const std:
     return comp;
 }
 
-inline void scale_table(std::vector<std::complex<double>> &tab, const std::vector<double> &comp)
+// Mean over the inputs m of output k, and over the outputs of input m, of |B_km|^2 - 1 for the
+// radix-R butterfly as the FP64 kernels compute it.
+struct ButterflyDeviation {
+    std::vector<double> row, col;
+};
+template <int R> inline ButterflyDeviation butterfly_deviation()
+{
+    ButterflyDeviation d{std::vector<double>(R, 0.0), std::vector<double>(R, 0.0)};
+    auto dev = [](double a, double b) { return (double)((long double)a * a + (long double)b * b - 1); };
+    using K = Roots<double>;
+    for (int m = 0; m < R; m++) {
+        double2 x[R];
+        for (int k = 0; k < R; k++) x[k] = make_double2(k == m ? 1.0 : 0.0, 0.0);
+        dft<R, +1>(x);
+        for (int k = 0; k < R; k++) {
+            double v;
+            if (R != 9) {
+                v = dev(x[k].x, x[k].y);  // constants, unrounded
+            } else {
+                // two 3-point butterflies and a root W9^(m1 r) between them: the constants' product
+                const int m1 = m % 3, r = k % 3, w = m1 * r;
+                const double d3 = dev(0.5, K::s3);
+                v = (r && m / 3 ? d3 : 0.0) + (m1 && k / 3 ? d3 : 0.0) +
+                    (w == 1 ? dev(K::c9, K::s9) : w == 2 ? dev(K::c9_2, K::s9_2) : w == 4 ? dev(K::c9_4, K::s9_4) : 0.0);
+            }
+            d.row[k] += v / R;
+            d.col[m] += v / R;
+        }
+    }
+    return d;
+}
+
+// The FP64 factors minus 1, from the roots of unity as the FP64 kernels hold them: r_p and
+// c_p are n (1 + O(1e-16)), so the network runs on the deviations to first order.
+inline std::vector<double> fp64_pair_deviation(const AxisPlan &pl, const std::vector<std::complex<double>> &tw)
+{
+    static const std::vector<ButterflyDeviation> devs = [] {
+        std::vector<ButterflyDeviation> d(17);
+        d[2] = butterfly_deviation<2>();
+        d[3] = butterfly_deviation<3>();
+        d[4] = butterfly_deviation<4>();
+        d[6] = butterfly_deviation<6>();
+        d[8] = butterfly_deviation<8>();
+        d[9] = butterfly_deviation<9>();
+        d[12] = butterfly_deviation<12>();
+        d[16] = butterfly_deviation<16>();
+        return d;
+    }();
+    const int n = pl.n;
+    std::vector<double> r(n, 0.0), c(n, 0.0);
+    for (int s = 0; s < pl.ns; s++) {
+        const int R = pl.radix[s], L = pl.len[s], q = L / R;
+        const ButterflyDeviation &B = devs[R];
+        for (int g0 = 0; g0 < n; g0 += L)
+            for (int j = 0; j < q; j++) {
+                double rm = 0, cm = 0;
+                for (int m = 0; m < R; m++) {
+                    rm += r[g0 + m * q + j];
+                    cm += c[g0 + m * q + j];
+                }
+                for (int k = 0; k < R; k++) {
+                    double w = 0;
+                    if (k) {
+                        const std::complex<double> &t = tw[(size_t)pl.twoff[s] + (size_t)(k - 1) * q + j];
+                        w = (double)((long double)t.real() * t.real() + (long double)t.imag() * t.imag() - 1);
+                    }
+                    r[g0 + k * q + j] = rm / R + B.row[k] + w;
+                    c[g0 + k * q + j] = cm / R + B.col[k] + w;
+                }
+            }
+    }
+    for (int p = 0; p < n; p++) r[p] = -0.5 * (r[p] + c[p]);
+    return r;
+}
+
+// Factors of the phase table's entries for the kernels of one precision.
+inline std::vector<long double> pair_compensation(bool fp64, const AxisPlan &pl, const std::vector<std::complex<double>> &tw)
+{
+    std::vector<long double> f(pl.n);
+    const std::vector<double> v = fp64 ? fp64_pair_deviation(pl, tw) : fp32_pair_compensation(pl, tw);
+    for (int p = 0; p < pl.n; p++) f[p] = fp64 ? 1.0L + v[p] : (long double)v[p];
+    return f;
+}
+
+inline void scale_table(std::vector<std::complex<long double>> &tab, const std::vector<long double> &comp)
 {
     for (size_t k = 0; k < tab.size(); k++) tab[k] *= comp[k];
 }

@@ -24,6 +24,7 @@
 namespace {
 
 using cd = std::complex<double>;
+using cl = std::complex<long double>;  // table entries, until they are rounded
 
 // Physical constants of the reference, DtypesConsts.cuh:55-57.
 constexpr double kPi = 3.14159265358979323846;
@@ -457,9 +458,20 @@ struct PassTimer {
     }
 };
 
-template <typename C> C to_c(const cd &v);
-template <> float2 to_c<float2>(const cd &v) { return make_float2((float)v.real(), (float)v.imag()); }
-template <> double2 to_c<double2>(const cd &v) { return make_double2(v.real(), v.imag()); }
+template <typename C, typename T> C to_c(const std::complex<T> &v)
+{
+    using S = decltype(C{}.x);
+    return C{(S)v.real(), (S)v.imag()};
+}
+
+// exp(i x): the double values, brought to modulus 1 (their rounding leaves up to 1e-16, the same
+// at every step).
+cl phase_factor(double x)
+{
+    const cd v = std::polar(1.0, x);
+    const long double c = v.real(), s = v.imag(), m = 1.5L - 0.5L * (c * c + s * s);
+    return cl(c * m, s * m);
+}
 
 // Tables of one configuration, gathered on the host and uploaded together, in stream order:
 // into what is left of the table area of the solver's memory block, else into an
@@ -468,7 +480,7 @@ template <> double2 to_c<double2>(const cd &v) { return make_double2(v.real(), v
 class TableSet {
 public:
     // table h, rounded to C, whose device address goes to *out at upload()
-    template <typename C> void add(const std::vector<cd> &h, void **out)
+    template <typename C, typename T> void add(const std::vector<std::complex<T>> &h, void **out)
     {
         const size_t at = bytes_.size();
         bytes_.resize(at + (sizeof(C) * (h.empty() ? 1 : h.size()) + 255) / 256 * 256);
@@ -570,22 +582,21 @@ bool encode_field_map(CUtensorMap *map, void *field, int nx, int ny, int nt, siz
 // factorised as (x factor)(y factor); fx = centred(i) / (dx nx).  crys[f] is the crystal
 // step (the y factor carries exp(-alpha dz / 2)), free[f] the free-space return; the
 // 1/(nx ny) normalisation is split as 1/nx, 1/ny (shipped 1/(nx ny nt) with OPO_ASIS_Q1).
-void diffraction_tables(const OpoParams &p, bool xa, const opo::AxisPlan &pl, std::vector<cd> crys[3],
-                        std::vector<cd> free[3])
+void diffraction_tables(const OpoParams &p, bool xa, const opo::AxisPlan &pl, std::vector<cl> crys[3],
+                        std::vector<cl> free[3])
 {
     const int n = pl.n;
     const double q1scale = (!xa && (p.flags & OPO_ASIS_Q1)) ? 1.0 / p.nt : 1.0;
     for (int f = 0; f < 3; f++) {
         const double d = xa ? p.dx : p.dy;
         const double c = 2 * kPi * kPi / p.kdiff[f] / (d * n) / (d * n);
-        crys[f].assign(n, cd(0, 0));
-        free[f].assign(n, cd(0, 0));
+        const long double loss = xa ? 1.0L : std::exp(-0.5L * (long double)p.alpha[f] * p.dz) * q1scale;
+        crys[f].assign(n, cl(0, 0));
+        free[f].assign(n, cl(0, 0));
         for (int pos = 0; pos < n; pos++) {
             const double u = centred(bin_of_position(pl, pos), n);
-            cd v = std::polar(1.0, -p.dz * c * u * u) / (double)n;
-            if (!xa) v *= std::exp(-0.5 * p.alpha[f] * p.dz) * q1scale;
-            crys[f][pos] = v;
-            free[f][pos] = std::polar(1.0, p.free_len * c * u * u) / (double)n;
+            crys[f][pos] = phase_factor(-p.dz * c * u * u) * (loss / n);
+            free[f][pos] = phase_factor(p.free_len * c * u * u) / (long double)n;
         }
     }
 }
@@ -902,12 +913,12 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
     set.add<C>(tw, &pc.tw);
     const bool phys = (p.flags & OPO_PHYSICS) != 0;
     const opo::AxisPlan &pl = pc.plan;
-    // FP32: every table of this plan carries the transform pair's gain compensation
-    const std::vector<double> comp = fp64 ? std::vector<double>() : opo::fp32_pair_compensation(pl, tw);
-    auto fix = [&](std::vector<cd> &t) {
-        if (!comp.empty()) opo::scale_table(t, comp);
+    // every table of this plan carries the transform pair's gain compensation
+    const std::vector<long double> comp = opo::pair_compensation(fp64, pl, tw);
+    auto fix = [&](std::vector<cl> &t) {
+        opo::scale_table(t, comp);
         if (pc.line_n && kind == kX) {  // the x bodies' table order (axis_line.cuh)
-            const std::vector<cd> pos = t;
+            const std::vector<cl> pos = t;
             const int rl = pl.radix[pl.ns - 1], ng = n / rl;
             for (int g0 = 0; g0 < ng; g0++)
                 for (int k = 0; k < rl; k++) t[(size_t)k * ng + g0] = pos[(size_t)g0 * rl + k];
@@ -919,13 +930,13 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
         // phase (the crystals compute b3, PPLN.cuh:73, but the reference never applies it)
         const double q2scale = (p.flags & OPO_ASIS_Q2) ? 1.0 / ((double)nx * ny) : 1.0;
         for (int f = 0; f < 3; f++) {
-            std::vector<cd> tab(nt);
+            const double b3 = (p.flags & OPO_TOD) ? p.beta3[f] : 0.0;
+            const long double loss = phys ? 1.0L : std::exp(-0.5L * (long double)p.alpha[f] * p.dz);
+            std::vector<cl> tab(nt);
             for (int pos = 0; pos < nt; pos++) {
                 const double wk = s->w[bin_of_position(pl, pos)];
-                const double b3 = (p.flags & OPO_TOD) ? p.beta3[f] : 0.0;
-                cd v = std::polar(1.0, p.dz * wk * (p.vinv[f] + 0.5 * wk * p.beta2[f] + wk * wk * b3 / 6.0));
-                if (!phys) v *= std::exp(-0.5 * p.alpha[f] * p.dz);
-                tab[pos] = v * (q2scale / nt);
+                tab[pos] = phase_factor(p.dz * wk * (p.vinv[f] + 0.5 * wk * p.beta2[f] + wk * wk * b3 / 6.0)) *
+                           (loss * q2scale / nt);
             }
             fix(tab);
             set.add<TT>(tab, &pc.tab[0][f]);
@@ -935,11 +946,11 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
         for (int f = 1; f < 3; f++) {
             const bool res = (p.resonant >> f) & 1u;
             const double R = f == 1 ? p.Rs : p.Ri;
-            const cd mirror = res ? std::sqrt(R) * std::polar(1.0, p.detuning) : cd(1, 0);
-            std::vector<cd> tab(nt);
+            const cl mirror = res ? std::sqrt((long double)R) * phase_factor(p.detuning) : cl(1, 0);
+            std::vector<cl> tab(nt);
             for (int pos = 0; pos < nt; pos++) {
                 const double wk = s->w[bin_of_position(pl, pos)];
-                tab[pos] = std::polar(1.0, 0.5 * wk * wk * p.gdd) * mirror / (double)nt;
+                tab[pos] = phase_factor(0.5 * wk * wk * p.gdd) * mirror / (long double)nt;
             }
             fix(tab);
             set.add<TT>(tab, &pc.tab[1][f]);
@@ -968,7 +979,7 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
             set.add<C>(e, &pc.eom);
         }
     } else {
-        std::vector<cd> crys[3], free[3];
+        std::vector<cl> crys[3], free[3];
         diffraction_tables(p, kind == kX, pl, crys, free);
         for (int f = 0; f < 3; f++) {
             fix(crys[f]);
@@ -1045,12 +1056,11 @@ template <typename C> int configure_plane(OpoSolver *s, int K, int threads, int 
     TableSet set;
     set.add<C>(twx, &pc.twx);
     set.add<C>(twy, &pc.twy);
-    std::vector<cd> crys[3], free[3];
-    // FP32: the same gain compensation as the separate x / y passes' tables
-    std::vector<double> comp;
-    if (!fp64) comp = opo::fp32_pair_compensation(pc.px, twx);
+    std::vector<cl> crys[3], free[3];
+    // the same gain compensation as the separate x / y passes' tables
+    std::vector<long double> comp = opo::pair_compensation(fp64, pc.px, twx);
     diffraction_tables(p, true, pc.px, crys, free);
-    for (int f = 0; f < 3 && !comp.empty(); f++) {
+    for (int f = 0; f < 3; f++) {
         opo::scale_table(crys[f], comp);
         opo::scale_table(free[f], comp);
     }
@@ -1059,8 +1069,8 @@ template <typename C> int configure_plane(OpoSolver *s, int K, int threads, int 
         set.add<TT>(free[f], &pc.tabx[1][f]);
     }
     diffraction_tables(p, false, pc.py, crys, free);
-    if (!fp64) comp = opo::fp32_pair_compensation(pc.py, twy);
-    for (int f = 0; f < 3 && !comp.empty(); f++) {
+    comp = opo::pair_compensation(fp64, pc.py, twy);
+    for (int f = 0; f < 3; f++) {
         opo::scale_table(crys[f], comp);
         opo::scale_table(free[f], comp);
     }
