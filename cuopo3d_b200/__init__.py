@@ -281,7 +281,7 @@ class Simulation:
                                           FILES_BINARY if binary else FILES_TEXT))
 
     def set_wait_limit(self, cycles):
-        """Bound of the warp-specialised passes' pipeline waits (SM cycles; 0: ~2 s)."""
+        """Bound of the TMA-fed passes' waits for their tiles (SM cycles; 0: ~2 s)."""
         self._check(lib().opo_set_wait_limit(self._h, int(cycles)))
 
     @property

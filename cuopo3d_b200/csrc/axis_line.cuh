@@ -181,7 +181,7 @@ template <typename C, bool X> inline size_t axis_line_smem(int n)
     }
 }
 
-// Whether the body for n points can be TMA-fed, and its columns per y box.
+// Whether the body for n points can be TMA-fed.
 template <typename C, bool X> inline bool axis_line_tma(int n)
 {
     switch (n) {
@@ -309,10 +309,10 @@ __device__ __forceinline__ void axis_line_tile(C *fp, unsigned lim, unsigned gs,
 
 // Brings the raw tile into sm with the TMA: x one bulk copy per line, y one tensor box (L
 // columns of N rows of the plane; columns past the grid read as zero).  Every thread returns
-// when the tile has landed; false when the bounded wait expired.
+// when the tile has landed; false when the bounded wait (wait clock cycles) expired.
 template <typename C, typename G>
 __device__ __forceinline__ bool axis_line_load(const C *fp, unsigned lim, const CUtensorMap *map, int c0, int plane, C *sm,
-                                               unsigned long long *bar)
+                                               unsigned long long *bar, long long wait)
 {
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
@@ -330,7 +330,7 @@ __device__ __forceinline__ bool axis_line_load(const C *fp, unsigned lim, const 
         }
     }
     __syncthreads();  // the barrier is initialised
-    return mbar_wait(bar, 0);
+    return mbar_wait(bar, 0, wait);
 }
 
 // First element and line count of tile `tile` of a line-specialised pass.

@@ -8,15 +8,14 @@
 
 namespace opo {
 
-// Tensor maps of the fields (y: boxes of L columns, N rows) and the error word of the passes'
-// bounded waits.
+// Tensor maps of the fields (y: boxes of L columns, N rows).
 struct AxisLineTma {
     CUtensorMap map[3];
 };
 
 // CTA u of a launch: tile u mod ntiles of the (u / ntiles)-th field of the mask.
 template <typename C, typename G, unsigned GS, bool TMA>
-__device__ __forceinline__ void axis_line_cta(const AxisArgs<C> &a, const CUtensorMap *maps, int *err)
+__device__ __forceinline__ void axis_line_cta(const AxisArgs<C> &a, const CUtensorMap *maps, int *err, long long wait)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     C *sm = reinterpret_cast<C *>(smem_raw);
@@ -35,9 +34,12 @@ __device__ __forceinline__ void axis_line_cta(const AxisArgs<C> &a, const CUtens
     if constexpr (TMA) {
         const unsigned hi = fdiv(a.g.tdiv, tile), lo = tile - hi * a.g.tdiv.d;
         unsigned long long *bar = reinterpret_cast<unsigned long long *>(smem_raw + G::BYTES);
-        if (!axis_line_load<C, G>(fp, lim, maps + f, (int)(lo * G::L * (sizeof(C) / 8)), (int)hi, sm, bar)) {
-            if (err) atomicExch(err, 101);
-            mbar_wait(bar, 0);  // the copy must not land in a later CTA's memory
+        if (!axis_line_load<C, G>(fp, lim, maps + f, (int)(lo * G::L * (sizeof(C) / 8)), (int)hi, sm, bar, wait)) {
+            // The host reports the error and takes the fields for lost.  The copy must not land
+            // in a later CTA's memory: this wait keeps the full bound.  (The threads that gave up go on
+            // with the others, which meet them at the tile's barriers.)
+            if (err) atomicExch(err, kAxisLineTimeout);
+            mbar_wait(bar, 0);
         }
     }
     axis_line_tile<C, G, G::THREADS, GS, TMA>(fp, lim, a.g.gs_j, tab, a.tw, sm);
@@ -46,13 +48,13 @@ __device__ __forceinline__ void axis_line_cta(const AxisArgs<C> &a, const CUtens
 template <typename C, typename G, unsigned GS>
 __global__ void __launch_bounds__(G::THREADS, G::MINB) axis_line_kernel(AxisArgs<C> a)
 {
-    axis_line_cta<C, G, GS, false>(a, nullptr, nullptr);
+    axis_line_cta<C, G, GS, false>(a, nullptr, nullptr, 0);
 }
 template <typename C, typename G, unsigned GS>
 __global__ void __launch_bounds__(G::THREADS, G::MINB)
-    axis_line_tma_kernel(AxisArgs<C> a, const __grid_constant__ AxisLineTma t, int *err)
+    axis_line_tma_kernel(AxisArgs<C> a, const __grid_constant__ AxisLineTma t, int *err, long long wait)
 {
-    axis_line_cta<C, G, GS, G::TMA>(a, t.map, err);
+    axis_line_cta<C, G, GS, G::TMA>(a, t.map, err, wait);
 }
 
 // Kernel of an axis of n points: square: the grid is, tma: TMA-fed (axis_line_tma).
@@ -80,7 +82,8 @@ template <typename C, bool X> const void *axis_line_func(int n, bool square, boo
 }
 
 template <typename C, bool X>
-cudaError_t launch_axis_line_t(const AxisArgs<C> &a, bool square, const CUtensorMap *maps, int *err, size_t smem, cudaStream_t st)
+cudaError_t launch_axis_line_t(const AxisArgs<C> &a, bool square, const CUtensorMap *maps, int *err, long long wait,
+                               size_t smem, cudaStream_t st)
 {
     int threads = 0;
     const void *fn = axis_line_func<C, X>(a.plan.n, square, maps != nullptr, &threads);
@@ -90,7 +93,8 @@ cudaError_t launch_axis_line_t(const AxisArgs<C> &a, bool square, const CUtensor
         void *args[] = {const_cast<AxisArgs<C> *>(&a)};
         return cudaLaunchKernel(fn, grid, dim3(threads), args, smem, st);
     }
-    void *args[] = {const_cast<AxisArgs<C> *>(&a), const_cast<CUtensorMap *>(maps), &err};
+    if (wait <= 0) wait = kWaitCycles;
+    void *args[] = {const_cast<AxisArgs<C> *>(&a), const_cast<CUtensorMap *>(maps), &err, &wait};
     return cudaLaunchKernel(fn, grid, dim3(threads), args, smem, st);
 }
 
@@ -107,8 +111,8 @@ template <typename C, bool X> cudaError_t configure_axis_line_t(int n)
 }
 
 #define OPO_AXIS_LINE_INSTANCE(C, X)                                                                \
-    template cudaError_t launch_axis_line_t<C, X>(const AxisArgs<C> &, bool, const CUtensorMap *, int *, size_t, \
-                                                  cudaStream_t);                                    \
+    template cudaError_t launch_axis_line_t<C, X>(const AxisArgs<C> &, bool, const CUtensorMap *, int *, long long, \
+                                                  size_t, cudaStream_t);                            \
     template cudaError_t configure_axis_line_t<C, X>(int);
 
 }  // namespace opo

@@ -344,9 +344,9 @@ struct OpoSolver {
     size_t table_left = 0;
     PassCfg pass[3];
     PlaneCfg plane;
-    int *err_dev = nullptr;  // error word of the warp-specialised passes
-    long long wait_cycles = 0;  // bound of their ring waits (0: the default ~2 s)
-    // Set when a warp-specialised pass gave up a wait: that pass's tiles were not all
+    int *err_dev = nullptr;  // error word of the TMA-fed passes
+    long long wait_cycles = 0;  // bound of their waits (0: the default ~2 s)
+    // Set when one of them gave up a wait: that pass's tiles were not all
     // written, so the fields are lost.  Cleared once all four fields have been uploaded
     // again (reloaded: bit per field) or initialised (opo_init_fields).
     bool fields_lost = false;
@@ -403,8 +403,9 @@ int cuda_fail(OpoSolver *s, cudaError_t e, const char *what)
         if (e_ != cudaSuccess) return cuda_fail((s), e_, what); \
     } while (0)
 
-// After a synchronisation with the solver's stream: a warp-specialised pass that gave up
-// on a bounded wait left a code in the error word (cleared here).
+// After a synchronisation with the solver's stream: a TMA-fed pass (warp-specialised, or an x- or
+// y-pass of a line body) that gave up on a bounded wait left a code in the error word
+// (cleared here).
 int check_pass_error(OpoSolver *s)
 {
     if (!s->err_dev) return OPO_OK;
@@ -414,16 +415,16 @@ int check_pass_error(OpoSolver *s)
     cudaMemset(s->err_dev, 0, sizeof(int));
     s->fields_lost = true;
     s->reloaded = 0;
-    return fail(s, OPO_ERR_CUDA, "a warp-specialised pass stopped after a pipeline wait timed out (code " +
-                                     std::to_string(code) + "); the fields are lost until all four are uploaded "
-                                     "again or initialised");
+    return fail(s, OPO_ERR_CUDA, std::string(code == opo::kAxisLineTimeout ? "an x- or y-pass" : "a warp-specialised pass") +
+                                     " gave up after its wait for a tile timed out (code " + std::to_string(code) +
+                                     "); the fields are lost until all four are uploaded again or initialised");
 }
 
 // Calls that read or advance the fields fail while they are lost (see fields_lost).
 int require_fields(OpoSolver *s)
 {
     if (!s->fields_lost) return OPO_OK;
-    return fail(s, OPO_ERR_CUDA, "the fields were lost when a warp-specialised pass gave up a pipeline wait; "
+    return fail(s, OPO_ERR_CUDA, "the fields were lost when a pass gave up its wait for a tile; "
                                  "upload all four (opo_set_field) or initialise them (opo_init_fields)");
 }
 
@@ -1224,8 +1225,8 @@ template <typename C> int enqueue_axis(OpoSolver *s, int kind, int which_tab, un
         const bool square = s->p.nx == s->p.ny;
         const CUtensorMap *maps = pc.line_tma ? pc.maps : nullptr;
         const cudaError_t e = kind == kX
-                                  ? opo::launch_axis_line_t<C, true>(a, square, maps, s->err_dev, pc.smem, s->stream)
-                                  : opo::launch_axis_line_t<C, false>(a, square, maps, s->err_dev, pc.smem, s->stream);
+                                  ? opo::launch_axis_line_t<C, true>(a, square, maps, s->err_dev, s->wait_cycles, pc.smem, s->stream)
+                                  : opo::launch_axis_line_t<C, false>(a, square, maps, s->err_dev, s->wait_cycles, pc.smem, s->stream);
         OPO_CU(s, e, "axis-pass launch");
     } else {
         OPO_CU(s, opo::launch_axis<C>(a, pc.v, kind == kX, pc.grid, pc.smem, s->stream), "axis-pass launch");
@@ -1883,7 +1884,7 @@ static int create_impl(const OpoParams *p, const double *w, const opo::PassVaria
             break;
         }
         const size_t fbytes = (s->esz * s->V + 255) / 256 * 256;
-        // partial sums, the three sums, the error word of the warp-specialised passes
+        // partial sums, the three sums, the error word of the TMA-fed passes
         s->sum_blocks = 148 * 4;
         const size_t nsum = 3 * ((size_t)s->sum_blocks + 1), sbytes = (sizeof(double) * nsum + sizeof(int) + 255) / 256 * 256;
         constexpr size_t kTableArea = 256 * 1024;

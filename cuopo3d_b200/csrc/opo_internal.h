@@ -272,10 +272,12 @@ template <typename C> cudaError_t launch_axis(const AxisArgs<C> &a, PassVariant 
 // y-pass then compiles its row stride in).  configure_axis_line allows its kernels the full
 // shared memory.
 // maps: TMA-fed, y from these tensor maps of the three fields (x ignores them); null: loads
-// through registers.  err: error word of the TMA waits.
+// through registers.  err: error word of the TMA waits (kAxisLineTimeout: one gave up), wait:
+// their bound in clock cycles (0: the default).
+constexpr int kAxisLineTimeout = 101;
 template <typename C, bool X>
-cudaError_t launch_axis_line_t(const AxisArgs<C> &a, bool square, const CUtensorMap *maps, int *err, size_t smem,
-                               cudaStream_t st);
+cudaError_t launch_axis_line_t(const AxisArgs<C> &a, bool square, const CUtensorMap *maps, int *err, long long wait,
+                               size_t smem, cudaStream_t st);
 template <typename C, bool X> cudaError_t configure_axis_line_t(int n);
 // x then y line pass of a square grid in one launch (axis_plane.cu), n points a side;
 // configure_axis_plane allows its kernel the full shared memory where it needs it.

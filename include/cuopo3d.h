@@ -318,12 +318,13 @@ const char *opo_noalloc_last_error(void);
  * has no counterpart: it is the denominator of the t-pass's FP64-pipe roofline. */
 int opo_fp64_peak(double *tflops);
 
-/* Waits for the solver's stream.  OPO_ERR_CUDA when a warp-specialised pass gave up one
- * of its bounded pipeline waits: its tiles were not all written, so the fields are lost
+/* Waits for the solver's stream.  OPO_ERR_CUDA when a pass that brings its tiles in with
+ * TMA (the warp-specialised ones; x- and y-passes of axes with a compiled body, from 128
+ * points on) gave up one of its bounded waits: the fields are then lost
  * and every call that reads or advances them fails until all four have been uploaded again
  * (opo_set_field) or initialised (opo_init_fields). */
 int opo_synchronize(OpoSolver *s);
-/* Bound of the warp-specialised passes' pipeline waits in SM clock cycles (0: the default,
+/* Bound of those passes' waits in SM clock cycles (0: the default,
  * about 2 s).  A short bound makes a pass give up and report OPO_ERR_CUDA instead of
  * waiting; it exists to exercise that error path.  The final drain of copies already
  * issued keeps the default bound.  No counterpart in the reference. */
