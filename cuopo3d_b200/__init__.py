@@ -24,6 +24,8 @@ DISPERSION, DIFFRACTION, PHYSICS, ASIS_Q1, ASIS_Q2, TOD = 1, 2, 4, 8, 16, 32
 FP32, FP64 = 0, 1
 # added to a t-pass "r1" in a tuning: the line-specialised t-pass (OPO_TUNE_LINE)
 LINE = 256
+# and beside it: a plane-wave solver's whole crystal in one launch (OPO_TUNE_WAVE)
+WAVE = 512
 PPLN_ID, MGOSPPLT_ID, MGOPPLN_ID, ZGP_ID = 0, 1, 2, 3
 CRYSTALS = {"ppln": PPLN_ID, "mgospplt": MGOSPPLT_ID, "mgosplt": MGOSPPLT_ID, "mgoppln": MGOPPLN_ID,
             "zgp": ZGP_ID}

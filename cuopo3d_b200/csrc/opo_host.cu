@@ -604,6 +604,12 @@ void diffraction_tables(const OpoParams &p, bool xa, const opo::AxisPlan &pl, st
 
 template <typename C> bool tpass_line_body(const OpoParams &p, opo::PassVariant v);
 
+// A single time line and no diffraction: the plane-wave kernel's grids.
+bool plane_wave(const OpoParams &p)
+{
+    return p.nx == 1 && p.ny == 1 && !(p.flags & (OPO_DIFFRACTION | OPO_ASIS_Q2));
+}
+
 // Default variant and tile size of a pass kind: the line t-pass where the grid has a body
 // (128 x 128 x 256: FP32 70 against 105 us, FP64 124 against 223 us), otherwise 96 KB of
 // shared memory for the three fields (4096 complex64 or 2048 complex128 per field), 256
@@ -612,9 +618,10 @@ void default_variant(const OpoParams &p, int kind, opo::PassVariant &v, size_t &
 {
     const bool fp64 = p.precision == OPO_FP64;
     const opo::PassVariant line{128, opo::kLineForm | (fp64 ? 4 : 16)};
-    const bool wave = p.nx == 1 && p.ny == 1 && !(p.flags & (OPO_DIFFRACTION | OPO_ASIS_Q2));
+    const bool wave = plane_wave(p);
     if (kind == kT && (wave || (fp64 ? tpass_line_body<double2>(p, line) : tpass_line_body<float2>(p, line)))) {
         v = line;
+        if (wave) v.r1 |= opo::kWaveForm;
         te = fp64 ? 1024 : 2048;
         return;
     }
@@ -694,12 +701,11 @@ template <typename C> bool use_tpass_line(const OpoParams &p, PassCfg &pc, std::
     return true;
 }
 
-// Whether a solver's crystal runs as one launch of the plane-wave kernel under t-setting v: a
-// single time line and no diffraction.  (The other settings, and a batch, keep the t-pass.)
+// Whether a solver's crystal runs as one launch of the plane-wave kernel under t-setting v.  (The
+// other settings, and a batch, keep the t-pass.)
 bool wave_setting(const OpoSolver *s, opo::PassVariant v)
 {
-    const OpoParams &p = s->p;
-    return opo::is_line(v) && !s->batched && p.nx == 1 && p.ny == 1 && !(p.flags & (OPO_DIFFRACTION | OPO_ASIS_Q2));
+    return opo::is_line(v) && (v.r1 & opo::kWaveForm) && !s->batched && plane_wave(s->p);
 }
 
 // Plan, cluster size and geometry of the plane-wave kernel; false when none fits (the t-pass
@@ -1581,7 +1587,7 @@ template <typename C> int autotune(OpoSolver *s)
         {
             // a compiled body or the plane-wave kernel: ahead of every generic and warp-specialised
             // variant on its grids, nothing to time
-            const opo::PassVariant lv{128, (fp64 ? 4 : 16) | opo::kLineForm};
+            const opo::PassVariant lv{128, (fp64 ? 4 : 16) | opo::kLineForm | (plane_wave(s->p) ? opo::kWaveForm : 0)};
             bool line = kind == kT && (wave_setting(s, lv) || opo::line_setting_only(s->p.nt)) &&
                         configure_pass<C>(s, kind, lv, tes[1]) == OPO_OK &&
                         (s->pass[kind].wave_K || s->pass[kind].line_nt);

@@ -164,7 +164,7 @@ struct WsArgs {
 // stage may use follows from the precision and CTA size (max_radix()).
 struct PassVariant {
     int threads;  // 128 or 256; 160 or 288: warp-specialised (128 / 256 consumers + a producer warp)
-    int r1;       // 4, 8 or 16, plus kLineForm for the line-specialised t-pass
+    int r1;       // 4, 8 or 16, plus kLineForm for the line-specialised t-pass (and kWaveForm)
 };
 
 // Flag in PassVariant::r1 (and in the r1 entries of the C-ABI tuning arrays): the
@@ -175,6 +175,10 @@ struct PassVariant {
 // with the fallback radix: the variant's radix in FP32, radix 4 (the register form) in
 // FP64.
 constexpr int kLineForm = 256;
+// Flag beside kLineForm: a 1 x 1 grid without diffraction runs its whole crystal as the plane-wave
+// kernel (wave_pass.cu), which a batch has no form of.  A flag of its own, so that a slot and a
+// standalone solver under the same line setting run the same t-pass, to the same bits.
+constexpr int kWaveForm = 512;
 inline int line_pixels(bool fp64) { return fp64 ? 4 : 8; }  // nx multiple of a line setting
 inline bool is_line(PassVariant v) { return (v.r1 & kLineForm) != 0; }
 inline int radix_of(PassVariant v) { return v.r1 & (kLineForm - 1); }

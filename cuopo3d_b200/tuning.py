@@ -21,7 +21,7 @@ def generic_t(precision, tuning):
     t = dict(tuning["t"])
     if not t["r1"] & LINE:
         return tuning
-    t["r1"] = 4 if precision == FP64 else t["r1"] - LINE
+    t["r1"] = 4 if precision == FP64 else t["r1"] & (LINE - 1)
     return {**tuning, "t": t}
 
 

@@ -269,9 +269,12 @@ int opo_set_tuning(OpoSolver *s, const int tuning[9]);
  * its size and the fallback radix (FP32: the given radix, FP64:
  * 4).  x- and y-passes whose axis length has a compiled body (16, 24, 32, 36, 48, 64, 72, 96,
  * 108, 128, 144, 192, 216, 256, 384, 512) run it under every setting of 128 or 256 threads;
- * such a setting's tile and radix then matter to other lengths only.  No counterpart in
+ * such a setting's tile and radix then matter to other lengths only.  OPO_TUNE_WAVE added
+ * as well runs the whole crystal of a plane-wave solver (nx = ny = 1 without diffraction; it
+ * starts so) in one launch; elsewhere, and in a batch, it changes nothing.  No counterpart in
  * the reference. */
 #define OPO_TUNE_LINE 256
+#define OPO_TUNE_WAVE 512
 int opo_get_tuning(const OpoSolver *s, int out[9]);
 
 /* Diffraction operator as one fused plane pass (Solver3D.cuh:282-323 applied at :954 and
