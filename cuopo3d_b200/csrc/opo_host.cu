@@ -357,7 +357,7 @@ struct OpoSolver {
     void *staging = nullptr;  // conversion buffer (V complex of the other precision)
     // captured launches: a round trip, the run's last round trip, a single pass
     cudaGraphExec_t graph_rt[3] = {nullptr, nullptr, nullptr};
-    bool single_ran = false;  // a single pass ran since the graphs were dropped
+    int singles = 0;  // single passes launched kernel by kernel since the graphs were dropped
     int rt_index = 0;
     long long launches = 0;
     int launches_rt[3] = {0, 0, 0};
@@ -541,7 +541,7 @@ void drop_graphs(OpoSolver *s)
             cudaGraphExecDestroy(g);
             g = nullptr;
         }
-    s->single_ran = false;
+    s->singles = 0;
 }
 
 // cuTensorMapEncodeTiled from the driver, looked up once through the runtime.
@@ -1426,15 +1426,19 @@ template <typename C> int run_graph(OpoSolver *s, int gi)
     return OPO_OK;
 }
 
-// A solver's first single pass is launched kernel by kernel (a graph of one use costs more
-// than its launches), later ones as a graph: 32 x 32 x 64 FP64, x and y apart (151 launches), 0.86
-// -> 0.60 ms a pass, three solvers in turn 0.41 -> 0.29 ms each; now 101 launches and 0.25 ms.
+// A solver's first two single passes are launched kernel by kernel, later ones as a graph.
+// B200: capturing, instantiating and first launching the graph takes 0.15-0.65 ms in the call
+// that does it, and each call after it saves 0.1-0.6 ms of launches (32 x 32 x 64 FP64, 101 launches:
+// 0.75 ms direct, 0.93 with the capture, 0.55 as a graph, each waited for; 96 x 96 x 192 FP32: 7.46,
+// 7.71, 6.92 ms): two passes lose about what the graph costs, so that no number of passes takes
+// much longer than it would with the better form throughout.  A plane wave's pass is one
+// launch already.
 template <typename C> int run_single_pass(OpoSolver *s)
 {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     OPO_CU(s, cudaStreamIsCapturing(s->stream, &cap), "capture status");
-    if (s->timing || !s->single_ran || cap != cudaStreamCaptureStatusNone) {
-        s->single_ran = true;
+    if (s->timing || s->singles < 2 || s->pass[kT].wave_K || cap != cudaStreamCaptureStatusNone) {
+        s->singles++;
         return enqueue_single_pass<C>(s);
     }
     return run_graph<C>(s, 2);
