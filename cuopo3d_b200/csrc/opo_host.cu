@@ -474,6 +474,12 @@ cl phase_factor(double x)
     return cl(c * m, s * m);
 }
 
+bool is_capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone;
+}
+
 // Tables of one configuration, gathered on the host and uploaded together, in stream order:
 // into what is left of the table area of the solver's memory block, else into an
 // allocation of their own (a cudaMalloc / cudaFree pair takes 55 us up to 64 KB and 700 us
@@ -500,7 +506,13 @@ public:
             OPO_CU(s, cudaMalloc(&mem, bytes_.size()), "cudaMalloc(tables)");
             allocs.push_back(mem);
         }
-        OPO_CU(s, cudaMemcpyAsync(mem, bytes_.data(), bytes_.size(), cudaMemcpyHostToDevice, s->stream), "copy(tables)");
+        // while the caller captures the stream the copy must not become a node of that graph
+        if (is_capturing(s->stream)) {
+            OPO_CU(s, cudaMemcpy(mem, bytes_.data(), bytes_.size(), cudaMemcpyHostToDevice), "copy(tables)");
+            OPO_CU(s, cudaStreamSynchronize(nullptr), "copy(tables)");
+        } else {
+            OPO_CU(s, cudaMemcpyAsync(mem, bytes_.data(), bytes_.size(), cudaMemcpyHostToDevice, s->stream), "copy(tables)");
+        }
         for (auto &sl : slots_) *sl.first = static_cast<char *>(mem) + sl.second;
         return OPO_OK;
     }
@@ -1435,9 +1447,7 @@ template <typename C> int run_graph(OpoSolver *s, int gi)
 // launch already.
 template <typename C> int run_single_pass(OpoSolver *s)
 {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    OPO_CU(s, cudaStreamIsCapturing(s->stream, &cap), "capture status");
-    if (s->timing || s->singles < 2 || s->pass[kT].wave_K || cap != cudaStreamCaptureStatusNone) {
+    if (s->timing || s->singles < 2 || s->pass[kT].wave_K || is_capturing(s->stream)) {
         s->singles++;
         return enqueue_single_pass<C>(s);
     }
@@ -1915,7 +1925,8 @@ static int create_impl(const OpoParams *p, const double *w, const opo::PassVaria
         s->err_dev = reinterpret_cast<int *>(s->partials + nsum);
         s->table_area = m + 4 * fbytes + sbytes;
         s->table_left = bytes - 4 * fbytes - sbytes;
-        if ((e = cudaMemsetAsync(s->mem, 0, 4 * fbytes + sbytes, s->stream)) != cudaSuccess) {
+        if ((e = is_capturing(s->stream) ? cudaMemset(s->mem, 0, 4 * fbytes + sbytes)
+                                         : cudaMemsetAsync(s->mem, 0, 4 * fbytes + sbytes, s->stream)) != cudaSuccess) {
             rc = cuda_fail(s, e, "memset");
             break;
         }
