@@ -1567,6 +1567,31 @@ template <typename C> int autotune(OpoSolver *s)
                 return configure_plane<C>(s, e.plane[0], e.plane[1], e.plane[2]);
             }
     }
+    TuneEntry best{key, {}, {}, {0, 256, 8}};
+    const size_t tes[3] = {fp64 ? 512u : 1024u, fp64 ? 1024u : 2048u, fp64 ? 2048u : 4096u};
+    const int threads[4] = {128, 256, 160, 288};  // 160 / 288: warp-specialised
+    const int r1s[3] = {4, 8, 16};
+    const long long launches0 = s->launches;
+    // Passes with nothing to time: a compiled body or the plane-wave kernel, ahead of every generic
+    // and warp-specialised variant on its grids, or no pass at all.
+    bool fixed[3];
+    for (int kind = 0; kind < 3; kind++) {
+        fixed[kind] = kind != kT && !(s->p.flags & OPO_DIFFRACTION);
+        best.v[kind] = s->pass[kind].v;
+        best.te[kind] = s->pass[kind].te;
+        if (fixed[kind]) continue;
+        const opo::PassVariant lv{128, (fp64 ? 4 : 16) | opo::kLineForm | (plane_wave(s->p) ? opo::kWaveForm : 0)};
+        bool line = kind == kT && (wave_setting(s, lv) || opo::line_setting_only(s->p.nt)) &&
+                    configure_pass<C>(s, kind, lv, tes[1]) == OPO_OK &&
+                    (s->pass[kind].wave_K || s->pass[kind].line_nt);
+        for (int r1 : {8, 4})
+            if (!line && configure_pass<C>(s, kind, opo::PassVariant{128, r1}, tes[1]) == OPO_OK)
+                line = (s->pass[kind].line_n || s->pass[kind].line_nt) && s->pass[kind].v.r1 == r1;
+        fixed[kind] = line;
+        if (!line) continue;
+        best.v[kind] = s->pass[kind].v;
+        best.te[kind] = tes[1];
+    }
     // The candidates are timed on scratch fields (zeroed, so no non-finite values), not on
     // the caller's: the fields are left as they were, as on a cache hit.  The guard puts
     // the caller's fields back and frees the scratch on every way out.
@@ -1582,37 +1607,21 @@ template <typename C> int autotune(OpoSolver *s)
             cudaFree(mem);
         }
     } scratch{s};
-    OPO_CU(s, cudaMalloc(&scratch.mem, 4 * s->esz * s->V), "cudaMalloc(autotune scratch fields)");
-    OPO_CU(s, cudaMemsetAsync(scratch.mem, 0, 4 * s->esz * s->V, s->stream), "memset(autotune scratch)");
-    for (int k = 0; k < 4; k++) {
-        scratch.saved[k] = s->field[k];
-        s->field[k] = static_cast<char *>(scratch.mem) + k * s->esz * s->V;
+    if (!fixed[kT] || !fixed[kX] || !fixed[kY]) {
+        OPO_CU(s, cudaMalloc(&scratch.mem, 4 * s->esz * s->V), "cudaMalloc(autotune scratch fields)");
+        OPO_CU(s, cudaMemsetAsync(scratch.mem, 0, 4 * s->esz * s->V, s->stream), "memset(autotune scratch)");
+        for (int k = 0; k < 4; k++) {
+            scratch.saved[k] = s->field[k];
+            s->field[k] = static_cast<char *>(scratch.mem) + k * s->esz * s->V;
+        }
     }
-    TuneEntry best{key, {}, {}, {0, 256, 8}};
-    const size_t tes[3] = {fp64 ? 512u : 1024u, fp64 ? 1024u : 2048u, fp64 ? 2048u : 4096u};
-    const int threads[4] = {128, 256, 160, 288};  // 160 / 288: warp-specialised
-    const int r1s[3] = {4, 8, 16};
-    const long long launches0 = s->launches;
     for (int kind = 0; kind < 3; kind++) {
         float best_ms = 1e30f;
-        best.v[kind] = s->pass[kind].v;
-        best.te[kind] = s->pass[kind].te;
-        if (kind != kT && !(s->p.flags & OPO_DIFFRACTION)) continue;
-        {
-            // a compiled body or the plane-wave kernel: ahead of every generic and warp-specialised
-            // variant on its grids, nothing to time
-            const opo::PassVariant lv{128, (fp64 ? 4 : 16) | opo::kLineForm | (plane_wave(s->p) ? opo::kWaveForm : 0)};
-            bool line = kind == kT && (wave_setting(s, lv) || opo::line_setting_only(s->p.nt)) &&
-                        configure_pass<C>(s, kind, lv, tes[1]) == OPO_OK &&
-                        (s->pass[kind].wave_K || s->pass[kind].line_nt);
-            for (int r1 : {8, 4})
-                if (!line && configure_pass<C>(s, kind, opo::PassVariant{128, r1}, tes[1]) == OPO_OK)
-                    line = (s->pass[kind].line_n || s->pass[kind].line_nt) && s->pass[kind].v.r1 == r1;
-            if (line) {
-                best.v[kind] = s->pass[kind].v;
-                best.te[kind] = tes[1];
-                continue;
-            }
+        if (fixed[kind]) {
+            // again on the scratch, whose addresses its tensor maps then hold
+            int rc = scratch.mem ? configure_pass<C>(s, kind, best.v[kind], best.te[kind]) : OPO_OK;
+            if (rc) return rc;
+            continue;
         }
         for (size_t te : tes)
             for (int th : threads)
@@ -1658,9 +1667,9 @@ template <typename C> int autotune(OpoSolver *s)
     }
     s->launches = launches0;
     // back on the caller's fields: configure the chosen passes again, so that the tensor
-    // maps of the warp-specialised kernels address those fields, not the scratch
+    // maps address those fields, not the scratch
     OPO_CU(s, cudaStreamSynchronize(s->stream), "autotune sync");
-    for (int k = 0; k < 4; k++) s->field[k] = scratch.saved[k];
+    for (int k = 0; k < 4 && scratch.mem; k++) s->field[k] = scratch.saved[k];
     for (int k = 0; k < 3; k++) {
         int rc = configure_pass<C>(s, k, best.v[k], best.te[k]);
         if (rc) return rc;

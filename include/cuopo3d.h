@@ -240,13 +240,14 @@ int opo_run_round_trips_tallied(OpoSolver *s, int n, double *tallies, int *done)
 int opo_set_pass_timing(OpoSolver *s, int enable);
 int opo_pass_times(OpoSolver *s, double ms[4], long long counts[4]);
 
-/* Time every compiled kernel variant (CTA size, first-stage radix) and tile size of
- * the t-, x- and y-passes on this solver's grid and keep the fastest for each, then
- * time the tuned x + y passes against every fused plane-pass variant (cluster size,
- * CTA size, first-stage radix) and keep the faster diffraction operator; results
+/* Choose the configuration for this solver's grid.  A pass whose axis has a compiled body
+ * takes it (opo_set_tuning).  For the others, time every compiled kernel variant (CTA size,
+ * first-stage radix) and tile size and keep the fastest; unless both x and y have bodies, then
+ * time these passes against every fused plane-pass variant (cluster size,
+ * CTA size, first-stage radix) and keep the faster diffraction operator.  Results
  * are cached per (grid, precision, device) for the process, so later solvers of the same
- * shape reuse them without timing.  The candidates are timed on temporary scratch fields
- * (4 x nx ny nt complex values, allocated for the call), so the solver's own fields are
+ * shape reuse them without timing.  Candidates are timed on temporary scratch fields
+ * (4 x nx ny nt complex values, allocated for the call when there is anything to time), so the solver's own fields are
  * left as they were whether or not the cache held the grid.  Stands in for the
  * reference's compile-time block sizes (DtypesConsts.cuh:48-50). */
 int opo_autotune(OpoSolver *s);
