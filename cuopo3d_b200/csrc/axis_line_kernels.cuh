@@ -69,7 +69,9 @@ template <typename C, bool X> const void *axis_line_func(int n, bool square, boo
         if constexpr (G::TMA) {                                                                     \
             if (tma && square) return reinterpret_cast<const void *>(axis_line_tma_kernel<C, G, SQ>); \
             if (tma) return reinterpret_cast<const void *>(axis_line_tma_kernel<C, G, 0u>);         \
-            return X ? nullptr : reinterpret_cast<const void *>(axis_line_kernel<C, G, 0u>);        \
+            /* y rows off 16 bytes; an x line is always fed by TMA */                               \
+            if constexpr (X) return nullptr;                                                        \
+            else return reinterpret_cast<const void *>(axis_line_kernel<C, G, 0u>);                 \
         } else {                                                                                    \
             if (square) return reinterpret_cast<const void *>(axis_line_kernel<C, G, SQ>);          \
             return reinterpret_cast<const void *>(axis_line_kernel<C, G, 0u>);                      \
