@@ -7,10 +7,10 @@
 // after the other, left the pass waiting on global memory (45 / 50 us for x / y in FP32,
 // 99 / 102 us in FP64 against 31 / 62 us of HBM at the measured rate).  The diffraction
 // factors do not couple the fields, so a tile here is L lines of one field: a third of the
-// shared memory and one load phase per tile, 8 (FP32, 64-80 registers) or 8 (FP64, 64-thread
-// CTAs at 128 registers) of them per SM whose phases overlap, every index and stride but the
-// y-pass's row stride a constant (and that one too on square grids).  128 x 128 x 256,
-// B200: FP32 x / y 37 / 35 us, FP64 65 / 71 us (6.2 / 5.6 TB/s); 256 x 256 x 512 FP32
+// shared memory and one load phase per tile, 8 (FP32 x, 64 registers), 7 (FP32 y, 72) or 8
+// (FP64, 64-thread CTAs at 128 registers) of them per SM whose phases overlap, every index and
+// stride but the y-pass's row stride a constant (and that one too on square grids).  128 x 128 x
+// 256, B200: FP32 x / y 39 / 40 us, FP64 70 / 79 us (5.7 / 5.1 TB/s); 256 x 256 x 512 FP32
 // 350 / 387 -> 245 / 285 us.
 //
 // Stages of a tile, all threads on one stage at a time: the RA-point stage from global
@@ -83,8 +83,10 @@ __host__ __device__ constexpr bool axis_plane(bool fp64, int n) { return n <= (f
 // 31.7.  From 64 points on two planes per SM are needed (64 x 64 x 64 FP64 22.5 -> 23.9 alone;
 // 64 x 64 x 128 40.0 / 28.8 -> 38.9 / 25.9), and in FP32, whose CTAs a plane's six stages keep
 // longer than the x and y tiles, all planes resident at once, four per SM (64 x 64 x 128 25.0 /
-// 16.3 -> 24.4 / 15.4; x 256 41.9 / 32.3 -> 43.5 / 31.2).  FP32 72 and 96 points: alone 5 and 9 %
-// slower at 256 samples, no body.
+// 16.3 -> 24.4 / 15.4; x 256 41.9 / 32.3 -> 43.5 / 31.2).  On 64 points and the nine time axes from
+// 64 to 256 samples, alone: inside the rule FP32 gains 2-6 % (108 samples loses 6), FP64 -2 to +6;
+// outside it 4-7 % are lost (96 samples, 288 planes, gains 3 and 9).  FP32 72 and 96 points: alone
+// 5 and 9 % slower at 256 samples, no body.
 inline bool axis_plane_pays(bool fp64, int n, unsigned planes)
 {
     return axis_plane(fp64, n) && (n <= 48 || (planes >= 2 * 148 && (fp64 || planes <= 4 * 148)));
@@ -150,7 +152,8 @@ template <typename C, bool X_, int N_> struct AxisLine {
     // TMA-fed: one item per thread, and from 128 points on -- loads through registers hold their
     // bytes in flight in L1, which beside the t-pass's shared memory (three solvers in turn, the
     // SMs' split at its largest) is 28 KB: 128 x 128 x 256 FP32 15.0 -> 14.0 ms a round trip, FP64
-    // 30.3 -> 27.7; alone, and below 128 points, the two are within 1-5 %, registers ahead
+    // 30.3 -> 27.7; alone, and below 128 points, the two are within 1-5 %, registers ahead.  (At 384
+    // and 512 points only FP64 x has one item per thread.)
     static constexpr bool TMA = ITEMS <= THREADS && N >= 128;
     // Registers: FP32 80 (at 64 the radix-16 y-pass of ragged grids spills: 47 us against 39),
     // FP64 128 with a radix above 8, else 96.

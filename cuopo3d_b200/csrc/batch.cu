@@ -1,5 +1,5 @@
 // Batched split-step: many OPO instances (uneven grids and parameters) advance together,
-// one persistent launch per pass covering the tiles of every instance.
+// one launch per pass and kernel body covering the tiles of every instance that it runs.
 //
 // Each instance lives in a slot that owns a single-instance solver (its resident
 // fields, FFT plans and phase tables, built with the batch's kernel variants).  The

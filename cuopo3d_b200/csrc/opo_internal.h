@@ -179,7 +179,7 @@ constexpr int kLineForm = 256;
 // kernel (wave_pass.cu), which a batch has no form of.  A flag of its own, so that a slot and a
 // standalone solver under the same line setting run the same t-pass, to the same bits.
 constexpr int kWaveForm = 512;
-inline int line_pixels(bool fp64) { return fp64 ? 4 : 8; }  // nx multiple of a line setting
+inline int line_pixels(bool fp64) { return fp64 ? 4 : 8; }  // nx multiple of a line setting (from its first, row-wise tiles)
 inline bool is_line(PassVariant v) { return (v.r1 & kLineForm) != 0; }
 inline int radix_of(PassVariant v) { return v.r1 & (kLineForm - 1); }
 // Line-specialised t-pass kernels: CTA size and the radix of the generic fallback.

@@ -81,7 +81,8 @@ typedef struct OpoConfig {
     double lp, ls;                     /* pump, signal wavelength (um); li = ls lp/(ls-lp) */
     int nx, ny, nt, nz;                /* grid; nz slices, dz = Lcr/(nz-1); nx = ny = 1 without
                                           OPO_DIFFRACTION is the plane-wave 1-D solver
-                                          (Solver1D.cuh), nt up to one tile per CTA;
+                                          (Solver1D.cuh), nt up to one tile per CTA, or to
+                                          the plane-wave kernel's cluster (opo_set_tuning);
                                           nx ny nt <= 2^31 - 1                           */
     double dQ;                         /* um/V; <= 0 keeps the crystal's 2 d33/pi          */
     double alpha[3];                   /* 1/um; < 0 keeps the crystal's value              */
@@ -323,8 +324,8 @@ const char *opo_noalloc_last_error(void);
 int opo_fp64_peak(double *tflops);
 
 /* Waits for the solver's stream.  OPO_ERR_CUDA when a pass that brings its tiles in with
- * TMA (the warp-specialised ones; x- and y-passes of axes with a compiled body, from 128
- * points on) gave up one of its bounded waits: the fields are then lost
+ * TMA (the warp-specialised ones; x- and y-passes of axes with a compiled body of 128 to 256
+ * points, in FP64 x to 512) gave up one of its bounded waits: the fields are then lost
  * and every call that reads or advances them fails until all four have been uploaded again
  * (opo_set_field) or initialised (opo_init_fields). */
 int opo_synchronize(OpoSolver *s);
@@ -339,10 +340,10 @@ long long opo_kernel_launches(const OpoSolver *s);
 const char *opo_last_error(const OpoSolver *s);
 const char *opo_version(void);
 
-/* ---- batched form: many instances, one persistent launch per pass ----------------- */
+/* ---- batched form: many instances, one launch per pass and kernel body ------------ */
 
 /* A batch advances every admitted instance (uneven grids and parameters, one slot
- * each) by whole cavity round trips, with one persistent kernel launch per pass for all
+ * each) by whole cavity round trips, with one kernel launch per pass and kernel body for all
  * of them and each round trip replayed as one CUDA graph.  Instances are admitted while
  * their device memory fits the HBM budget; all instances of a batch take the same
  * number of z-steps.  The reference runs one instance per process (cuOPO3D.sh:65-86
