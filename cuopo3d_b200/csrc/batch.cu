@@ -303,6 +303,7 @@ thread_local std::string g_batch_err;
 
 int bfail(OpoBatch *b, int code, const std::string &msg)
 {
+    if (code == OPO_ERR_CUDA || code == OPO_ERR_NOMEM) (void)cudaGetLastError();  // reported here, not by the next launch
     if (b) b->err = msg;
     else g_batch_err = msg;
     return code;

@@ -393,6 +393,7 @@ int fail(OpoSolver *s, int code, const std::string &msg)
 
 int cuda_fail(OpoSolver *s, cudaError_t e, const char *what)
 {
+    (void)cudaGetLastError();  // reported here, not once more by the next launch
     return fail(s, e == cudaErrorMemoryAllocation ? OPO_ERR_NOMEM : OPO_ERR_CUDA,
                 std::string(what) + ": " + cudaGetErrorString(e));
 }

@@ -36,7 +36,10 @@ extern "C" int opo_fp64_peak(double *tflops)
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return OPO_ERR_CUDA;
     double *buf = nullptr;
-    if (cudaMalloc(&buf, 4 * sizeof(double)) != cudaSuccess) return OPO_ERR_NOMEM;
+    if (cudaMalloc(&buf, 4 * sizeof(double)) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return OPO_ERR_NOMEM;
+    }
     const double h[3] = {0.9999999, 1e-9, 1.0};
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     int rc = OPO_OK;
