@@ -591,6 +591,21 @@ bool encode_field_map(CUtensorMap *map, void *field, int nx, int ny, int nt, siz
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The tensor maps through which a pass reads the solver's fields (t: Api, Ap, As, Ai; y: Ap, As,
+// Ai): boxes of a line body's columns or a warp-specialised tile's lines.
+bool encode_pass_maps(const OpoSolver *s, int kind, PassCfg &pc)
+{
+    const OpoParams &p = s->p;
+    const unsigned px = (pc.line_tma ? (unsigned)pc.geo.nlines : pc.wsa.px) * (unsigned)(s->esz / 8);
+    const unsigned lines = pc.line_tma ? (unsigned)p.ny : pc.wsa.box_lines;
+    const int first = kind == kT ? 0 : 1;
+    for (int k = first; k < 4; k++)
+        if (!encode_field_map(&pc.maps[k - first], s->field[k], p.nx, p.ny, p.nt, s->esz, px, kind == kT ? 1 : lines,
+                              kind == kT ? lines : 1))
+            return false;
+    return true;
+}
+
 // Diffraction factor tables of the x axis (xa) or the y axis in the digit-reversed order
 // of plan pl: the propagator exp(sign L 2 pi^2 / k (fx^2 + fy^2)) of Solver3D.cuh:282-323
 // factorised as (x factor)(y factor); fx = centred(i) / (dx nx).  crys[f] is the crystal
@@ -678,10 +693,7 @@ template <typename C> void use_axis_line(const OpoSolver *s, bool xa, PassCfg &p
     // (x lines always are); a batch's kernels load through registers
     pc.line_tma = !s->batched && (xa ? opo::axis_line_tma<C, true>(n)
                                      : opo::axis_line_tma<C, false>(n) && (size_t)p.nx * sizeof(C) % 16 == 0);
-    if (pc.line_tma && !xa)
-        for (int f = 0; f < 3; f++)
-            pc.line_tma = pc.line_tma && encode_field_map(&pc.maps[f], s->field[f + 1], p.nx, p.ny, p.nt, sizeof(C),
-                                                          L * (unsigned)(sizeof(C) / 8), (unsigned)n, 1);
+    if (pc.line_tma && !xa) pc.line_tma = encode_pass_maps(s, kY, pc);
     if (pc.line_tma) pc.smem += 16;  // the mbarrier
 }
 
@@ -888,12 +900,7 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
             w.lines = lines;
             w.box_lines = bl;
             w.field_bytes = (unsigned)(lines * px * es);
-            const unsigned b0 = px * w.inner_mult;
-            const int first = kind == kT ? 0 : 1;  // t-pass maps Api, Ap, As, Ai; y-pass Ap, As, Ai
-            for (int k = first; k < 4; k++)
-                if (!encode_field_map(&pc.maps[k - first], s->field[k], nx, ny, nt, es, b0, kind == kT ? 1 : bl,
-                                      kind == kT ? bl : 1))
-                    return fail(s, OPO_ERR_INVALID, "tensor map encoding failed");
+            if (!encode_pass_maps(s, kind, pc)) return fail(s, OPO_ERR_INVALID, "tensor map encoding failed");
         }
         pc.smem = opo::kWsHeaderBytes + w.nstages * (size_t)w.stage_bytes;
         if (pc.smem > 227 * 1024) return fail(s, OPO_ERR_INVALID, "stage ring does not fit in shared memory");
@@ -1604,6 +1611,10 @@ template <typename C> int autotune(OpoSolver *s)
         {
             if (!mem) return;
             for (int k = 0; k < 4; k++) s->field[k] = saved[k];
+            for (int kind : {kT, kY}) {  // after an error the last candidates' maps hold the scratch
+                PassCfg &pc = s->pass[kind];
+                if (pc.line_tma || (opo::is_ws(pc.v) && pc.wsa.mode == opo::kWsTensor && pc.wsa.box_lines)) encode_pass_maps(s, kind, pc);
+            }
             cudaStreamSynchronize(s->stream);
             cudaFree(mem);
         }
