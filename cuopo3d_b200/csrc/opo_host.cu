@@ -274,6 +274,12 @@ int bin_of_position(const opo::AxisPlan &p, int pos)
     }
     return bin;
 }
+std::vector<int> bins_of_plan(const opo::AxisPlan &p)
+{
+    std::vector<int> bin(p.n);
+    for (int pos = 0; pos < p.n; pos++) bin[pos] = bin_of_position(p, pos);
+    return bin;
+}
 
 // Centred index of FFT bin i on an n-point grid after the reference's fftshift
 // (EFields3D.cuh:141-171): (i + n/2) mod n - n/2.
@@ -615,17 +621,18 @@ void diffraction_tables(const OpoParams &p, bool xa, const opo::AxisPlan &pl, st
                         std::vector<cl> free[3])
 {
     const int n = pl.n;
+    const std::vector<int> bin = bins_of_plan(pl);
     const double q1scale = (!xa && (p.flags & OPO_ASIS_Q1)) ? 1.0 / p.nt : 1.0;
     for (int f = 0; f < 3; f++) {
         const double d = xa ? p.dx : p.dy;
         const double c = 2 * kPi * kPi / p.kdiff[f] / (d * n) / (d * n);
-        const long double loss = xa ? 1.0L : std::exp(-0.5L * (long double)p.alpha[f] * p.dz) * q1scale;
+        const long double inv = 1.0L / n, scale = xa ? inv : std::exp(-0.5L * (long double)p.alpha[f] * p.dz) * q1scale * inv;
         crys[f].assign(n, cl(0, 0));
         free[f].assign(n, cl(0, 0));
         for (int pos = 0; pos < n; pos++) {
-            const double u = centred(bin_of_position(pl, pos), n);
-            crys[f][pos] = phase_factor(-p.dz * c * u * u) * (loss / n);
-            free[f][pos] = phase_factor(p.free_len * c * u * u) / (long double)n;
+            const double u = centred(bin[pos], n);
+            crys[f][pos] = phase_factor(-p.dz * c * u * u) * scale;
+            free[f][pos] = phase_factor(p.free_len * c * u * u) * inv;
         }
     }
 }
@@ -955,15 +962,15 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
         // dispersion exp(i dz w (vinv + w b2/2)) exp(-alpha dz/2) / nt (Solver3D.cuh:153-169,
         // with the 1/nt of the inverse transform folded in); OPO_TOD adds w^3 b3/6 to the
         // phase (the crystals compute b3, PPLN.cuh:73, but the reference never applies it)
+        const std::vector<int> bin = bins_of_plan(pl);
         const double q2scale = (p.flags & OPO_ASIS_Q2) ? 1.0 / ((double)nx * ny) : 1.0;
         for (int f = 0; f < 3; f++) {
             const double b3 = (p.flags & OPO_TOD) ? p.beta3[f] : 0.0;
-            const long double loss = phys ? 1.0L : std::exp(-0.5L * (long double)p.alpha[f] * p.dz);
+            const long double loss = phys ? 1.0L : std::exp(-0.5L * (long double)p.alpha[f] * p.dz), scale = loss * q2scale / nt;
             std::vector<cl> tab(nt);
             for (int pos = 0; pos < nt; pos++) {
-                const double wk = s->w[bin_of_position(pl, pos)];
-                tab[pos] = phase_factor(p.dz * wk * (p.vinv[f] + 0.5 * wk * p.beta2[f] + wk * wk * b3 / 6.0)) *
-                           (loss * q2scale / nt);
+                const double wk = s->w[bin[pos]];
+                tab[pos] = phase_factor(p.dz * wk * (p.vinv[f] + 0.5 * wk * p.beta2[f] + wk * wk * b3 / 6.0)) * scale;
             }
             fix(tab);
             set.add<TT>(tab, &pc.tab[0][f]);
@@ -973,11 +980,12 @@ template <typename C> int configure_pass(OpoSolver *s, int kind, opo::PassVarian
         for (int f = 1; f < 3; f++) {
             const bool res = (p.resonant >> f) & 1u;
             const double R = f == 1 ? p.Rs : p.Ri;
-            const cl mirror = res ? std::sqrt((long double)R) * phase_factor(p.detuning) : cl(1, 0);
+            const cl scale = (res ? std::sqrt((long double)R) * phase_factor(p.detuning) : cl(1, 0)) / (long double)nt;
             std::vector<cl> tab(nt);
             for (int pos = 0; pos < nt; pos++) {
-                const double wk = s->w[bin_of_position(pl, pos)];
-                tab[pos] = phase_factor(0.5 * wk * wk * p.gdd) * mirror / (long double)nt;
+                const double wk = s->w[bin[pos]];
+                const cl v = phase_factor(0.5 * wk * wk * p.gdd);
+                tab[pos] = res ? v * scale : v * scale.real();
             }
             fix(tab);
             set.add<TT>(tab, &pc.tab[1][f]);
