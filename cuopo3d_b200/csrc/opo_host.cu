@@ -1688,11 +1688,13 @@ template <typename C> int autotune(OpoSolver *s)
     s->launches = launches0;
     // back on the caller's fields: configure the chosen passes again, so that the tensor
     // maps address those fields, not the scratch
-    OPO_CU(s, cudaStreamSynchronize(s->stream), "autotune sync");
-    for (int k = 0; k < 4 && scratch.mem; k++) s->field[k] = scratch.saved[k];
-    for (int k = 0; k < 3; k++) {
-        int rc = configure_pass<C>(s, k, best.v[k], best.te[k]);
-        if (rc) return rc;
+    if (scratch.mem) {
+        OPO_CU(s, cudaStreamSynchronize(s->stream), "autotune sync");
+        for (int k = 0; k < 4; k++) s->field[k] = scratch.saved[k];
+        for (int k = 0; k < 3; k++) {
+            int rc = configure_pass<C>(s, k, best.v[k], best.te[k]);
+            if (rc) return rc;
+        }
     }
     if (int rc = configure_plane<C>(s, best.plane[0], best.plane[1], best.plane[2])) return rc;
     std::lock_guard<std::mutex> lock(g_tune_mu);
